@@ -241,6 +241,8 @@ gbfsm_status gbfsm_host_device_pointer(void *host, void **device) {
 
 int32_t gbfsm_lanes_warps_per_sm(void) { return lanes_warps_per_sm(); }
 
+int32_t gbfsm_lanes_stage_limit(void) { return lanes_stage_limit(); }
+
 gbfsm_status gbfsm_lanes_run(const gbfsm_automaton *table, int32_t n_automata,
                              const gbfsm_task *tasks, int32_t n_tasks, const uint8_t *data,
                              const int64_t *offsets, const gbfsm_chunk_io *chunk_io,

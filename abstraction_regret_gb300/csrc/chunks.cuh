@@ -74,6 +74,13 @@ __device__ __forceinline__ uint32_t byte_at(const uint8_t *p) { return __ldg(p);
 constexpr int kShiftWindow = 32;    // bytes a chunk start may move forward
 constexpr uint32_t kShiftSet = 4u;  // a two-byte superset this small ends the search
 
+// Size of the two-byte superset `key`, at most 255 where the automaton has the byte table
+// (its 64 KiB stay in L1; the rows are 256 KiB and take two loads).
+__device__ __forceinline__ uint32_t pair_size(const gbfsm_nfa_dev &A, uint32_t key) {
+    if (A.pair_size) return __ldg(A.pair_size + key);
+    return __ldg(A.pair_row + key + 1) - __ldg(A.pair_row + key);
+}
+
 // Start of a later chunk whose nominal bounds are [nb, ne) (input-relative). For an
 // automaton with a two-byte superset table the start moves forward to the first position
 // of its first min(kShiftWindow, (ne - nb) / 4) bytes whose superset has at most kShiftSet
@@ -84,22 +91,28 @@ __device__ __forceinline__ int64_t chunk_start(const gbfsm_nfa_dev &A, const uin
                                                int64_t nb, int64_t ne) {
     if (A.pair_row == nullptr) return nb;
     const int w = (int)min((int64_t)kShiftWindow, max((int64_t)1, (ne - nb) / 4));
+    // two positions at a time, their size loads in flight together: a warp waits for the
+    // longest of its 32 searches, but every further load is a random gather
     uint32_t prev = byte_at(base + nb - 2), cur = byte_at(base + nb - 1);
     int best = 0;
     uint32_t best_size = 0xffffffffu;
-    for (int t = 0; t < w; ++t) {
-        const uint32_t key = prev * 256u + cur;
-        const uint32_t size = __ldg(A.pair_row + key + 1) - __ldg(A.pair_row + key);
-        if (size <= kShiftSet) {
-            best = t;
-            break;
+    for (int t = 0; t < w && best_size > kShiftSet; t += 2) {
+        uint32_t size[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            size[u] = 0xffffffffu;
+            if (t + u < w) {
+                size[u] = pair_size(A, prev * 256u + cur);
+                prev = cur;
+                cur = byte_at(base + nb + t + u);
+            }
         }
-        if (size < best_size) {
-            best_size = size;
-            best = t;
-        }
-        prev = cur;
-        cur = byte_at(base + nb + t);
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (best_size > kShiftSet && size[u] < best_size) {
+                best_size = size[u];
+                best = t + u;
+            }
     }
     return nb + best;
 }

@@ -170,6 +170,47 @@ def lane_state_records(nfa):
     return recs.astype(np.uint32), ext.astype(np.uint32)
 
 
+def slot_table(nfa):
+    """The slot table of an epsilon-free NFA (csrc/slots.cu): a dict of ``slots``, ``pairs``
+    (uint32), ``state_code`` (uint32 [n]), ``sets`` (uint32 [k, 3]: code, list, size),
+    ``set_code``, ``accept_code`` and ``multi_code``; None when the automaton's wildcard
+    edges (256 entries each) make it far larger than its edges."""
+    n = int(nfa.num_states)
+    srp, tgt, sym = (np.ascontiguousarray(x, dtype=np.int32) for x in
+                     (nfa.sym_row_ptr, nfa.sym_targets, nfa.sym_symbols))
+    acc = np.ascontiguousarray(nfa.accept, dtype=np.uint8)
+    nnz = int(srp[-1])
+    cap = 4 * nnz + 4 * n + 4096
+    cap_pairs = 4 * nnz + 1024
+    slots = np.empty(cap, dtype=np.uint32)
+    pairs = np.empty(2 * cap_pairs, dtype=np.uint32)
+    codes = np.empty(n + 3 * (n // 4 + 64), dtype=np.uint32)
+    info = np.zeros(8, dtype=np.int64)
+    st = native.lib().gbfsm_slots_build(
+        n, srp.ctypes.data, tgt.ctypes.data if nnz else None, sym.ctypes.data if nnz else None,
+        acc.ctypes.data, cap, slots.ctypes.data, cap_pairs, pairs.ctypes.data, codes.size,
+        codes.ctypes.data, info.ctypes.data)
+    if st == native.UNSUPPORTED:
+        return None
+    native.check(st, "gbfsm_slots_build")
+    n_slots, n_pairs, set_code, accept_code, multi_code, n_sets = (int(x) for x in info[:6])
+    return {"slots": slots[:n_slots], "pairs": pairs[:2 * n_pairs], "state_code": codes[:n],
+            "sets": codes[n:n + 3 * n_sets].reshape(n_sets, 3), "set_code": set_code,
+            "accept_code": accept_code, "multi_code": multi_code}
+
+
+def narrow_slots(table) -> np.ndarray | None:
+    """A slot table's 3-byte form (uint8 bytes: labels, then 16-bit codes, then pairs, each
+    padded to 16 bytes); None when a code needs more than 16 bits."""
+    slots, pairs = table["slots"], table["pairs"]
+    if table["multi_code"] + 1 + pairs.size // 2 > 1 << 16:
+        return None
+    parts = [(slots & 0xFF).astype(np.uint8), (slots >> 8).astype(np.uint16),
+             pairs.astype(np.uint16)]
+    return np.concatenate([np.concatenate([p.view(np.uint8),
+                                           np.zeros(-p.nbytes % 16, np.uint8)]) for p in parts])
+
+
 class DeviceNFA:
     """An NFA (ours or gpufsm's, duck-typed on the CSR fields) resident on a GPU."""
 
@@ -247,31 +288,85 @@ class DeviceNFA:
         self.lanes = pairs is not None
         self.pair_sizes = np.diff(pairs[0]).astype(np.int32) if pairs is not None else None
         self.pair_mean = float(self.pair_sizes.mean()) if pairs is not None else float("inf")
-        lane = lane_state_records(nfa) if pairs is not None else None
-        if lane is None:
+        table = slot_table(nfa) if pairs is not None else None
+        lane = lane_state_records(nfa) if pairs is not None and table is None else None
+        self.stage, self.stage_bytes = native.LANE_STAGE_NONE, 0
+        if lane is None and table is None:
             pairs = None
             self.lanes = False
             self.pair_sizes, self.pair_mean = None, float("inf")
         if pairs is not None:
             prow, precs = pairs
-            tg = np.asarray(nfa.sym_targets, dtype=np.int64)
             with torch.cuda.device(dev):
-                self.edge_sym = _padded(max(1, nnz), 2, dev, torch.int16)
-                if nnz:
-                    self.edge_sym[:nnz].copy_(torch.from_numpy(
-                        np.ascontiguousarray(ssy, dtype=np.int16)))
                 self.pair_row = torch.from_numpy(np.ascontiguousarray(prow)).to(dev)
-                lane_states, lane_ext = lane
-                self.pair_lanes = _records(lane_states[precs[:, 0].astype(np.int64)], dev)
-                self.lane_edges = _records(lane_states[tg] if nnz else lane_states[:0], dev)
-                self.lane_labels_ext = torch.from_numpy(
-                    np.ascontiguousarray(lane_ext).view(np.int32).ravel()).to(dev)
-            d.edge_sym = self.edge_sym.data_ptr()
+                if table is not None:
+                    self._upload_slots(d, table, precs[:, 0], srp, nfa, dev)
+                else:
+                    self._upload_lane_records(d, lane, precs[:, 0], ssy, nfa, dev)
             d.pair_row = self.pair_row.data_ptr()
-            d.pair_lanes = self.pair_lanes.data_ptr()
-            d.lane_edges = self.lane_edges.data_ptr()
-            d.lane_labels_ext = self.lane_labels_ext.data_ptr()
         self.desc = d
+
+    def _upload_slots(self, d, table, pair_states, srp, nfa, dev) -> None:
+        """The slot table, the codes of the two-byte supersets and the state record of
+        every code; how the lane launch of a pool of this automaton alone may stage it."""
+        code, multi = table["state_code"], table["multi_code"]
+        n = self.num_states
+        ids = np.arange(n, dtype=np.int64)
+        row = np.asarray(srp, dtype=np.int64)
+        recs = np.zeros((multi, 4), dtype=np.uint32)
+        recs[code] = np.stack([ids, _info(nfa, ids), row[:-1], row[1:]], axis=1)
+        sets = table["sets"]
+        recs[sets[:, 0], 0] = sets[:, 1]
+        recs[sets[:, 0], 1] = native.CODE_SET
+        recs[sets[:, 0], 2] = sets[:, 2]
+
+        def put(a):
+            raw = np.ascontiguousarray(a).view(np.uint8).ravel()
+            buf = _padded(max(1, raw.size), 1, dev)
+            if raw.size:
+                buf[: raw.size].copy_(torch.from_numpy(raw))
+            return buf
+
+        self.slots = put(table["slots"])
+        self.slot_pairs = put(table["pairs"])
+        self.pair_codes = put(code[pair_states.astype(np.int64)])
+        self.code_recs = put(recs)
+        narrow = narrow_slots(table)
+        self.slot_narrow = put(narrow) if narrow is not None else None
+        d.slots = self.slots.data_ptr()
+        d.slot_pairs = self.slot_pairs.data_ptr()
+        d.slot_narrow = self.slot_narrow.data_ptr() if narrow is not None else None
+        self.pair_size = put(np.minimum(self.pair_sizes, 255).astype(np.uint8))
+        d.pair_codes = self.pair_codes.data_ptr()
+        d.pair_size = self.pair_size.data_ptr()
+        d.code_recs = self.code_recs.data_ptr()
+        d.num_slots = table["slots"].size
+        d.num_pairs = table["pairs"].size // 2
+        d.set_code, d.accept_code, d.multi_code = table["set_code"], table["accept_code"], multi
+        d.start_code = int(code[self.start_state])
+        limit = int(native.lib().gbfsm_lanes_stage_limit())
+        wide = -(-table["slots"].nbytes // 16) * 16 + -(-table["pairs"].nbytes // 16) * 16
+        if wide <= limit:
+            self.stage, self.stage_bytes = native.LANE_STAGE_WIDE, wide
+        elif narrow is not None and narrow.size <= limit:
+            self.stage, self.stage_bytes = native.LANE_STAGE_NARROW, int(narrow.size)
+
+    def _upload_lane_records(self, d, lane, pair_states, ssy, nfa, dev) -> None:
+        """Lane records of every edge's target and of the two-byte supersets' states."""
+        tg = np.asarray(nfa.sym_targets, dtype=np.int64)
+        nnz = self.num_sym_edges
+        self.edge_sym = _padded(max(1, nnz), 2, dev, torch.int16)
+        if nnz:
+            self.edge_sym[:nnz].copy_(torch.from_numpy(np.ascontiguousarray(ssy, dtype=np.int16)))
+        lane_states, lane_ext = lane
+        self.pair_lanes = _records(lane_states[pair_states.astype(np.int64)], dev)
+        self.lane_edges = _records(lane_states[tg] if nnz else lane_states[:0], dev)
+        self.lane_labels_ext = torch.from_numpy(
+            np.ascontiguousarray(lane_ext).view(np.int32).ravel()).to(dev)
+        d.edge_sym = self.edge_sym.data_ptr()
+        d.pair_lanes = self.pair_lanes.data_ptr()
+        d.lane_edges = self.lane_edges.data_ptr()
+        d.lane_labels_ext = self.lane_labels_ext.data_ptr()
 
     @property
     def edge_bytes(self) -> int:

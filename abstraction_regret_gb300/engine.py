@@ -344,6 +344,7 @@ class DevicePlan:
         io.aut_ids = self._d_aut.data_ptr() if self._d_aut is not None else None
         if task_count_word is not None:
             io.task_count = self._hdr(task_count_word)
+        io.lane_stage, io.lane_stage_bytes = self.engine.lane_stage
         return io
 
     def launch(self, data_ptr: int, d_off, d_ends, d_flags, d_lens, d_examined, stream,
@@ -366,6 +367,7 @@ class DevicePlan:
         io = self.chunk_io(None)
         launches = 0
         if lane_slices:
+            io.lane_share = len(lane_slices)
             fork = torch.cuda.Event()
             fork.record(stream)
             joins = []
@@ -528,6 +530,9 @@ class PersistentEngine:
             self.table = torch.from_numpy(raw).to(self.device)
             props = torch.cuda.get_device_properties(self.device)
         self.sm_count = props.multi_processor_count
+        # a pool of one NFA whose slot table fits: the lane launch stages it
+        self.lane_stage = ((self.dev[0].stage, self.dev[0].stage_bytes)
+                           if len(self.dev) == 1 and isinstance(self.dev[0], DeviceNFA) else (0, 0))
         with torch.cuda.device(self.device):
             self.lane_warps_per_sm = int(lib.gbfsm_lanes_warps_per_sm()) or LANE_WARPS_PER_SM
         self.resident_warps = self.sm_count * self.ctas_per_sm * (block_threads // 32)

@@ -31,6 +31,7 @@ NFA_HAS_ANY = 2
 EDGE_SYMBOL_MASK = 0x1FF
 EDGE_ACCEPT = 1 << 9
 EDGE_HAS_EPS = 1 << 10
+CODE_SET = 1 << 11  # GBFSM_CODE_SET
 
 FLAG_TIMEOUT = -1
 
@@ -60,6 +61,18 @@ class NfaDev(ctypes.Structure):
         ("pair_lanes", ctypes.c_void_p),
         ("lane_edges", ctypes.c_void_p),
         ("lane_labels_ext", ctypes.c_void_p),
+        ("slots", ctypes.c_void_p),
+        ("slot_pairs", ctypes.c_void_p),
+        ("slot_narrow", ctypes.c_void_p),
+        ("pair_codes", ctypes.c_void_p),
+        ("code_recs", ctypes.c_void_p),
+        ("pair_size", ctypes.c_void_p),
+        ("num_slots", ctypes.c_uint32),
+        ("num_pairs", ctypes.c_uint32),
+        ("set_code", ctypes.c_uint32),
+        ("accept_code", ctypes.c_uint32),
+        ("multi_code", ctypes.c_uint32),
+        ("start_code", ctypes.c_uint32),
     ]
 
 
@@ -123,8 +136,11 @@ class ChunkIO(ctypes.Structure):
     _fields_ = [("chunks", ctypes.c_void_p), ("records", ctypes.c_void_p),
                 ("overflow_tasks", ctypes.c_void_p), ("overflow_count", ctypes.c_void_p),
                 ("task_count", ctypes.c_void_p), ("n_chunks", ctypes.c_int32),
-                ("aut_ids", ctypes.c_void_p)]
+                ("aut_ids", ctypes.c_void_p), ("lane_stage", ctypes.c_int32),
+                ("lane_stage_bytes", ctypes.c_int32), ("lane_share", ctypes.c_int32)]
 
+
+LANE_STAGE_NONE, LANE_STAGE_WIDE, LANE_STAGE_NARROW = range(3)  # GBFSM_LANE_STAGE_*
 
 PLAN_MAX_SLICES = 16  # GBFSM_PLAN_MAX_SLICES
 
@@ -163,7 +179,7 @@ PLAN_SLICES = 16
 
 (TASK_WHOLE, TASK_CHUNK, TASK_FIXUP, TASK_LANES, TASK_DFA_GROUP, TASK_DFA_CHUNK,
  TASK_DFA_FIXUP) = range(7)
-LANE_CAPACITY = 4  # members a lane holds (kLaneSlots)
+LANE_CAPACITY = 4  # members a lane holds without a slot table (kLaneSlots)
 CHUNK_RECORD_BYTES = 256
 STATIC_SCRATCH_BYTES = 32 << 20  # GBFSM_STATIC_SCRATCH_BYTES
 CHUNK_DTYPE = [("input", "<i4"), ("index", "<i4"), ("begin", "<i8"), ("end", "<i8")]
@@ -211,6 +227,9 @@ SIGNATURES: dict[str, tuple] = {
     "gbfsm_lanes_run": (ctypes.c_int, [_vp, _i32, _vp, _i32, _vp, _vp, _P(ChunkIO), _vp]),
     "gbfsm_nfa_run_static": (ctypes.c_int, [_P(NfaDev), _vp, _vp, _i32, _P(Plan), _vp, _vp,
                                             _vp, _vp]),
+    "gbfsm_slots_build": (_i32, [_i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _i64, _vp,
+                                 _vp]),
+    "gbfsm_lanes_stage_limit": (_i32, []),
     "gbfsm_workload_walk": (_i32, [_i32, _vp, _vp, _vp, _vp, _i32, _vp, _i32, _u64, _vp, _i32]),
     "gbfsm_lanes_run_range": (ctypes.c_int, [_vp, _i32, _vp, _i32, _vp, _vp, _vp, _P(ChunkIO),
                                              _vp]),
@@ -228,7 +247,7 @@ SIGNATURES: dict[str, tuple] = {
                                             _P(ChunkIO), _i32, _vp, _vp, _vp, _vp, _vp]),
 }
 
-ABI_VERSION = 3
+ABI_VERSION = 4
 
 _lib: ctypes.CDLL | None = None
 

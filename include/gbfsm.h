@@ -37,7 +37,7 @@
 extern "C" {
 #endif
 
-#define GBFSM_ABI_VERSION 3
+#define GBFSM_ABI_VERSION 4
 #define GBFSM_ANY_SYMBOL 256 /* src/gpufsm/core/nfa.py:16 */
 #define GBFSM_WORD_BITS 64   /* src/gpufsm/core/packing.py:21 */
 
@@ -126,7 +126,29 @@ typedef struct gbfsm_nfa_dev {
     const gbfsm_lane_rec *pair_lanes;
     const gbfsm_lane_rec *lane_edges;
     const uint32_t *lane_labels_ext;
+    /* Optional (NULL = lanes use the records above): the slot table of gbfsm_slots_build,
+     * which lane chunks then use instead, with pair_row and, per entry of the two-byte
+     * supersets, the state's code (pair_codes). slot_pairs: two codes per pair;
+     * code_recs[code]: the state record (as first_edges) of the state of a code below
+     * multi_code; of a set, {its list's code, GBFSM_CODE_SET, its size, 0}. slot_narrow (NULL when a code needs more than 16 bits): the labels
+     * (uint8), then the codes (uint16), then the pairs (two uint16), each padded to 16
+     * bytes. Every array starts on a 16-byte boundary and is padded to 16 bytes. */
+    const uint32_t *slots;
+    const uint32_t *slot_pairs;
+    const void *slot_narrow;
+    const uint32_t *pair_codes;
+    const gbfsm_edge *code_recs;
+    /* Optional: min(size, 255) of every two-byte superset ([65536]; NULL = from pair_row) */
+    const uint8_t *pair_size;
+    uint32_t num_slots;
+    uint32_t num_pairs;
+    uint32_t set_code;    /* codes below are states that do not accept */
+    uint32_t accept_code; /* codes from here on accept, up to multi_code */
+    uint32_t multi_code;
+    uint32_t start_code;
 } gbfsm_nfa_dev;
+
+#define GBFSM_CODE_SET (1u << 11) /* info bit of a set's entry in code_recs */
 
 /* A DFA on the device. table[s * 256 + c] holds the successor of s on byte c in the low
  * bits and, in the top bit, whether that successor accepts; entries are 2 bytes when
@@ -325,7 +347,17 @@ typedef struct gbfsm_chunk_io {
                                      index is 0) */
     const int32_t *aut_ids;       /* per-input automaton (device, n_inputs), for LANES tasks
                                      with automaton -1 and DFA_GROUP tasks; NULL = all 0 */
+    int32_t lane_stage;           /* GBFSM_LANE_STAGE_*: the lane launch of a pool of one
+                                     automaton copies its slot table to shared memory */
+    int32_t lane_stage_bytes;     /* the bytes that takes (gbfsm_nfa_dev's slots and pairs, or
+                                     slot_narrow, each array padded to 16 bytes) */
+    int32_t lane_share;           /* lane launches that run side by side (slices of a batch,
+                                     each with its range); 0 or 1: this one alone */
 } gbfsm_chunk_io;
+
+#define GBFSM_LANE_STAGE_NONE 0
+#define GBFSM_LANE_STAGE_WIDE 1   /* slots and slot_pairs */
+#define GBFSM_LANE_STAGE_NARROW 2 /* slot_narrow */
 
 /* Scratch bytes for a persistent launch whose largest NFA has `max_words` set words. */
 size_t gbfsm_persistent_workspace_bytes(int32_t max_words, const gbfsm_plan *plan);
@@ -374,6 +406,23 @@ int32_t gbfsm_pageable_access(void);
  * No counterpart in the reference (which packs and copies every batch on the host). */
 gbfsm_status gbfsm_gather_inputs(const uint64_t *src_ptrs, const int64_t *offsets,
                                  int32_t n_inputs, uint8_t *dst, void *stream);
+
+/* Build the slot table of an epsilon-free NFA (host only, HOST arrays in the reference CSR
+ * layout; csrc/slots.cu has the layout): slots [cap_slots], pairs [2 * cap_pairs], codes
+ * [cap_codes]: the code of every state, then {code, list, members} of every set that has
+ * one (at most (cap_codes - num_states) / 3). info[0..5] receive the number of slots, of
+ * pairs, the codes where sets begin, where accepting states and sets begin and where they
+ * end (gbfsm_nfa_dev.set_code, accept_code, multi_code), and the number of sets.
+ * GBFSM_UNSUPPORTED when the table (wildcard edges count as 256) exceeds a capacity.
+ * No counterpart in the reference. */
+int32_t gbfsm_slots_build(int32_t num_states, const int32_t *sym_row_ptr,
+                          const int32_t *sym_targets, const int32_t *sym_symbols,
+                          const uint8_t *accept, int64_t cap_slots, uint32_t *slots,
+                          int64_t cap_pairs, uint32_t *pairs, int64_t cap_codes,
+                          uint32_t *codes, int64_t *info);
+
+/* Largest gbfsm_chunk_io.lane_stage_bytes of the lane launch on the current device. */
+int32_t gbfsm_lanes_stage_limit(void);
 
 /* Resident warps per SM of the lane launch on the current device (0 when it cannot run):
  * a batch whose LANES tasks fit sm_count times this runs in one wave. No counterpart in
