@@ -197,10 +197,12 @@ __global__ void __launch_bounds__(kMaxBlockThreads, kPersistMinBlocks) persisten
 
 int32_t persistent_ctas_query(const PersistLayout &L, const gbfsm_plan &p);
 
+// Opts the kernel in to the most shared memory any layout may take: the limit belongs to the
+// kernel, so setting it to one layout's size would lower it under an earlier, larger one.
 cudaError_t ensure_smem(size_t bytes) {
     if (bytes <= 48u * 1024u) return cudaSuccess;
     return cudaFuncSetAttribute(persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)bytes);
+                                smem_optin() - (int)kSmemReserve);
 }
 
 }  // namespace
