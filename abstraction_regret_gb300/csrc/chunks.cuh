@@ -261,44 +261,6 @@ __device__ inline void run_chunk(const gbfsm_nfa_dev &nfa, const Rows &R, WarpSc
 
 // ---- lane chunk (one chunk per thread; up to kLaneSlots states) ----------------------------
 
-// Sequential 4-byte words of a byte range starting at any alignment: aligned 16-byte
-// blocks read one block ahead (never past `end`), each word put together by one funnel
-// shift of two aligned words.
-struct WordStream {
-    const uint8_t *blk;
-    const uint8_t *end;
-    uint4 cur, nxt;
-    uint32_t wi;  // aligned word (0..3) of cur holding the next byte
-    uint32_t sh;  // 8 x the byte offset of the next byte in that word
-
-    __device__ __forceinline__ static uint32_t word(const uint4 &v, uint32_t i) {
-        return i == 0u ? v.x : i == 1u ? v.y : i == 2u ? v.z : v.w;
-    }
-
-    __device__ __forceinline__ void init(const uint8_t *p, const uint8_t *e) {
-        end = e;
-        const uint64_t a = reinterpret_cast<uint64_t>(p);
-        blk = reinterpret_cast<const uint8_t *>(a & ~15ull);
-        wi = (uint32_t)((a >> 2) & 3u);
-        sh = (uint32_t)(a & 3u) * 8u;
-        cur = ld_stream16(blk);
-        nxt = (blk + 16 < end) ? ld_stream16(blk + 16) : make_uint4(0, 0, 0, 0);
-    }
-
-    __device__ __forceinline__ uint32_t next_word() {
-        const uint32_t lo = word(cur, wi);
-        const uint32_t hi = wi == 3u ? nxt.x : word(cur, wi + 1u);
-        const uint32_t w = __funnelshift_r(lo, hi, sh);
-        if (++wi == 4u) {
-            wi = 0u;
-            blk += 16;
-            cur = nxt;
-            nxt = (blk + 16 < end) ? ld_stream16(blk + 16) : make_uint4(0, 0, 0, 0);
-        }
-        return w;
-    }
-};
-//
 // The set is kept as the lane records (gbfsm_lane_rec) of its members, slot q valid when
 // bit q of `valid` is set. Per byte: find each member's edges labelled with the byte --
 // two byte-wise compares of its packed labels for a state in the fast form, a scan of

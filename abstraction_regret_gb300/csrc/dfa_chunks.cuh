@@ -2,44 +2,39 @@
 // verdicts (dfa_chunks.cu, tasks GBFSM_TASK_DFA_CHUNK and GBFSM_TASK_DFA_FIXUP).
 //
 // A DFA walk is one dependent table lookup per byte, so a long input is a long chain. Cut
-// it into chunks. Chunk 0 walks exactly from the start state. A later chunk starting at
-// position b does not know its start state, so it walks the set of ALL states: after each
-// byte the set becomes the distinct successors of its members, and for a random DFA it
-// shrinks like 2n/t; once it holds a single state (position p, the collapse), every start
-// state leads there, so from p on the chunk's walk is the true walk, whatever came before.
-// The chunk records p, its first accept after p, its state at its end and -- continuing
-// that exact walk past its end into the next chunk -- the first accept of this overlap.
+// it into chunks and follow every state a chunk might start in. For a random DFA the set
+// of all n states shrinks like 2n/t after t bytes, so it is down to 16 members after about
+// n/8 bytes, where it takes 2n bytes to reach a single one. So:
+//
+// 1. Collapse (a warp per chunk): from the chunk's start b the set of all states is walked
+//    until it has at most kEntries members; its position p and the members, the chunk's
+//    entry states, go to its record. The first chunk instead walks its first bytes exactly
+//    from the start state: one entry state.
+// 2. Walk (kEntries lanes per chunk, a lane per entry state): from p through the chunk and
+//    on to the next chunk's p. Each lane records its state there and its first accept.
+//    Lanes whose states have met read the same table entries, which costs nothing more.
+// 3. Fix-up (a warp per input): the true state at the first chunk's p is known; it is one
+//    of the entry states of its chunk, whose record gives the state at the next chunk's p,
+//    and so on. The first accept on that path is the input's verdict.
+//
+// A chunk whose set never shrinks to kEntries members has no entry states: the chunk before
+// walks on through it (up to the automaton's dfa_overlap bytes past its own end). Where a
+// walk ends before the next entry position, the fix-up walks the gap.
+//
+// Early stop: an accept of the first chunk, or one found by every lane of a chunk, is in
+// the input's true walk whatever came before, so the input's verdict lies at or before it.
+// The chunk lowers the input's latch to its index, and chunks of a higher index, polling
+// the latch, stop (p = -2). The fix-up returns before it reads a stopped chunk.
+//
+// What bounds it. The walk: the latency of a dependent lookup through L2, 0.2 us a byte,
+// along a chunk. The collapse: about 2n ln(n/8) lookups a chunk, gathers of one table
+// column (2-byte entries 512 bytes apart) that the LSU takes one sector at a time. The
+// planner's chunk length balances the two. 8 inputs of 2 MiB on 8192 states: 3.1 ms
+// (collapse 1.5, walk 1.6, fix-up 0.06) against 29.7 ms when a chunk had to collapse to a
+// single state before its walk counted; 24 inputs of 0.5..4 MB on 16384 states 8.8 against
+// 71 ms; one of 1 MiB on 256 states 0.33 against 1.46 ms.
+//
 // Positions count the bytes consumed from the start of the input.
-//
-// The overlap is as long as the next chunk needs: a chunk publishes its collapse position
-// in its record as soon as it has it, and the previous chunk's overlap walk, polling that
-// word, stops once it has passed it (at once when the next chunk stopped early), and in
-// any case at the next chunk's end or after `overlap` bytes (the automaton's
-// dfa_overlap). When the next chunk never collapses, the overlap covers it whole and
-// records the true state at its end, so the fix-up need not walk it. A stale word (the
-// next chunk's task not started yet) can only cut an overlap short; the fix-up checks
-// every link against the final records, so verdicts never depend on the timing.
-//
-// Fix-up (one lane per input, serial over the input's chunks): the true state at each
-// chunk start is known from the previous chunk's record. Chunk k is linked when chunk
-// k-1's walk is exact (it is chunk 0 or it collapsed) and its overlap reached p_k: the
-// overlap is then the true walk over (b_k, p_k], so its first accept (if any) is the
-// input's next accept, and otherwise chunk k's record is exact from p_k on. A chunk that
-// is not linked has its gap (b_k, p_k], or the whole chunk if it never collapsed, walked
-// serially from the known true state. Verdicts are exactly those of a serial walk
-// (src/gpufsm/reference.py:68-81).
-//
-// Set walk of a chunk, by one warp: while the set has more than 32 members it is a bitmap
-// of the states in shared memory (each lane scans its words, looks up the successors of
-// their members and sets their bits with shared atomics); then one member per lane,
-// duplicates removed with __match_any_sync, until one lane is left.
-//
-// Early stop: an accept found by chunk 0's walk, by a collapsed chunk's walk or by its
-// overlap is in the input's true walk, so the input's verdict lies at or before it. The
-// chunk lowers the input's latch to its index (the overlap: to the next chunk's index),
-// and every chunk of a higher index, polling the latch, stops (p = -2). The fix-up never
-// reads a stopped chunk: it returns at the latching chunk or earlier. It would walk one
-// whole, as a chunk that never collapsed.
 #pragma once
 
 #include "common.cuh"
@@ -48,19 +43,19 @@
 
 namespace gbfsm {
 
-// Record of a DFA chunk: the first 32 bytes of its GBFSM_CHUNK_RECORD_BYTES record slot.
+constexpr int kEntries = 16;  // entry states of a chunk: two chunks walk in a warp
+
+// Record of a DFA chunk, in its GBFSM_CHUNK_RECORD_BYTES record slot.
 struct DfaChunkRecord {
-    int32_t p;        // collapse position (0 for an input's first chunk), -1: none,
-                      // -2: stopped, kPending while the set walk runs
-    int32_t acc;      // first accept in (p, end], -1: none (first chunk: in [0, end])
-    int32_t end_state;
-    int32_t ov_len;   // bytes walked past the chunk end (exact when p >= 0)
-    int32_t ov_acc;   // first accept in the overlap, -1: none
-    int32_t ov_state; // the state at the end of the overlap (when ov_acc < 0)
-    int32_t pad[2];
+    int32_t p;      // entry position; -1: the set stayed larger, -2: stopped
+    int32_t at;     // the same, but never -2 (the chunk before reads it while this one walks)
+    int32_t count;  // entry states
+    int32_t done;   // position the lanes walked to
+    uint16_t entry[kEntries];
+    uint16_t exit[kEntries];  // each lane's state at `done`, when it has not accepted
+    int32_t acc[kEntries];    // first accept in (p, done], -1: none (first chunk: in [0, p] too)
 };
-static_assert(sizeof(DfaChunkRecord) == 32 && sizeof(DfaChunkRecord) <= GBFSM_CHUNK_RECORD_BYTES,
-              "DFA chunk record slot");
+static_assert(sizeof(DfaChunkRecord) <= GBFSM_CHUNK_RECORD_BYTES, "DFA chunk record slot");
 
 __device__ __forceinline__ DfaChunkRecord *dfa_record(void *records, int32_t chunk) {
     return reinterpret_cast<DfaChunkRecord *>(static_cast<uint8_t *>(records) +
@@ -69,8 +64,7 @@ __device__ __forceinline__ DfaChunkRecord *dfa_record(void *records, int32_t chu
 
 __device__ __forceinline__ const DfaChunkRecord *dfa_record(const void *records,
                                                             int32_t chunk) {
-    return reinterpret_cast<const DfaChunkRecord *>(static_cast<const uint8_t *>(records) +
-                                                    (size_t)chunk * GBFSM_CHUNK_RECORD_BYTES);
+    return dfa_record(const_cast<void *>(records), chunk);
 }
 
 template <typename Entry>
@@ -81,7 +75,8 @@ __device__ __forceinline__ uint32_t dfa_entry(const Entry *T, uint32_t s, uint32
 constexpr int kLatchPollBytes = 256;  // serial steps between two polls of the latch
 constexpr int kLatchPollSets = 16;    // light bitmap steps between two polls
 constexpr int kPollEveryStep = 512;   // set size above which every bitmap step polls
-constexpr int32_t kPending = -3;      // a record's p while its chunk's set walk runs
+constexpr int kMeetBytes = 4;  // bytes between two removals of members that have met
+constexpr int kListMembers = 1024;    // members from which a set is kept as a list
 
 // True when a chunk of index below `index` has latched the input (latch may be NULL).
 __device__ __forceinline__ bool latched_below(const int32_t *latch, int32_t index) {
@@ -97,36 +92,13 @@ __device__ __forceinline__ bool warp_latched_below(const int32_t *latch, int32_t
     return v < index;
 }
 
-// One lane: consume bytes [a, b) of `base` from state s. Returns the state at b, or at the
-// first accepting position q in (a, b], which goes to `acc` (-1 when none). With a latch,
-// polls it every kLatchPollBytes bytes and returns early with `stopped` set once a chunk
-// below `index` has latched.
 template <typename Entry>
-__device__ uint32_t dfa_span(const Entry *T, uint32_t s, const uint8_t *base, int64_t a,
-                             int64_t b, int64_t &acc, const int32_t *latch = nullptr,
-                             int32_t index = 0, bool *stopped = nullptr) {
-    constexpr uint32_t ACC = EntryTraits<Entry>::kAccept;
-    acc = -1;
-    if (b <= a) return s;
-    ByteStream bs;
-    bs.init(base + a, b - a);
-    for (int64_t q0 = a; q0 < b; q0 += kLatchPollBytes) {
-        if (latched_below(latch, index)) {
-            *stopped = true;
-            return s;
-        }
-        const int64_t q1 = min(b, q0 + (int64_t)kLatchPollBytes);
-        for (int64_t q = q0; q < q1; ++q) {
-            const uint32_t e = dfa_entry(T, s, bs.next());
-            s = e & ~ACC;
-            if (e & ACC) {
-                acc = q + 1;
-                return s;
-            }
-        }
+struct GlobalEntries {
+    const Entry *T;
+    __device__ __forceinline__ uint32_t operator()(uint32_t s, uint32_t c) const {
+        return dfa_entry(T, s, c);
     }
-    return s;
-}
+};
 
 __device__ __forceinline__ int32_t warp_sum_i32(int32_t v) {
 #pragma unroll
@@ -135,242 +107,351 @@ __device__ __forceinline__ int32_t warp_sum_i32(int32_t v) {
 }
 
 // The whole warp: walk the set of all n states from position b over bytes [b, e) until it
-// holds one state. Returns the collapse position (the state in `sigma`, every lane), -1
-// when the set still has two or more members at e, or -2 when a chunk below `index` has
-// latched the input (latch may be NULL). bm0 / bm1: shared bitmaps of at least
-// ceil(n / 32) words; list: 32 shared words.
+// has at most `want` (<= 32) members. Returns that position (lane l < count holds a member
+// in `member`), -1 when the set is still larger at e, or -2 when a chunk below `index` has
+// latched the input (latch may be NULL). bm0 / bm1: shared bitmaps of at least ceil(n / 32)
+// words; list: 2 * kListMembers shared 16-bit words. The set is a bitmap while it is large,
+// then a list (a step then costs a lookup, an atomic and a ballot per 32 members, whatever
+// n; scanning the bitmap for 64 members of 8192 states took 10 times the instructions),
+// then a member per lane.
 template <typename Entry>
 __device__ int64_t dfa_collapse(const Entry *T, uint32_t n, const uint8_t *base, int64_t b,
-                                int64_t e, uint32_t *bm0, uint32_t *bm1, uint32_t *list,
-                                uint32_t &sigma, const int32_t *latch, int32_t index) {
+                                int64_t e, int want, uint32_t *bm0, uint32_t *bm1,
+                                uint16_t *list, uint32_t &member, int32_t &count,
+                                const int32_t *latch, int32_t index) {
     constexpr uint32_t ACC = EntryTraits<Entry>::kAccept;
     const uint32_t lane = lane_id();
     const uint32_t nw = (n + 31u) >> 5;
+    count = 0;
+    member = 0;
     if (e <= b) return -1;
-    // first byte: the successors of every state
-    for (uint32_t w = lane; w < nw; w += 32) bm1[w] = 0u;
-    __syncwarp();
-    {
-        const uint32_t c = __ldg(base + b);
-        for (uint32_t s = lane; s < n; s += 32) {
-            const uint32_t t = dfa_entry(T, s, c) & ~ACC;
-            atomicOr(bm1 + (t >> 5), 1u << (t & 31u));
-        }
-    }
-    __syncwarp();
-    int64_t pos = b + 1;
-    uint32_t *cur = bm1, *nxt = bm0;
-    int32_t count = 0;
-    for (uint32_t w = lane; w < nw; w += 32) count += __popc(cur[w]);
-    count = warp_sum_i32(count);
-    // many members: bitmaps
-    while (count > 32 && pos < e) {
-        if ((count > kPollEveryStep || (pos - b) % kLatchPollSets == 0) &&
-            warp_latched_below(latch, index))
-            return -2;
-        const uint32_t c = __ldg(base + pos);
-        for (uint32_t w = lane; w < nw; w += 32) nxt[w] = 0u;
+    int64_t pos = b;
+    uint32_t polls = 0;
+    ByteStream bytes;
+    if (n <= 32u) {  // every state, one per lane
+        count = (int32_t)n;
+        member = lane < n ? lane : 0xffffffffu;
+    } else {
+        // first byte: the successors of every state
+        for (uint32_t w = lane; w < nw; w += 32) bm1[w] = 0u;
         __syncwarp();
-        for (uint32_t w = lane; w < nw; w += 32) {
-            uint32_t bits = cur[w];
-            while (bits) {  // up to four lookups in flight per lane
-                uint32_t s4[4];
-                int k = 0;
+        {
+            const uint32_t c = __ldg(base + b);
+            for (uint32_t s0 = lane; s0 < n; s0 += 32 * 8) {  // eight lookups in flight
+                uint32_t t[8];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (bits) {
-                        s4[u] = (w << 5) + (uint32_t)(__ffs(bits) - 1);
-                        bits &= bits - 1u;
-                        k = u + 1;
-                    }
-                }
-                uint32_t t4[4];
+                for (int u = 0; u < 8; ++u)
+                    if (s0 + 32u * u < n) t[u] = dfa_entry(T, s0 + 32u * u, c) & ~ACC;
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (u < k) t4[u] = dfa_entry(T, s4[u], c) & ~ACC;
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (u < k) atomicOr(nxt + (t4[u] >> 5), 1u << (t4[u] & 31u));
+                for (int u = 0; u < 8; ++u)
+                    if (s0 + 32u * u < n) atomicOr(bm1 + (t[u] >> 5), 1u << (t[u] & 31u));
             }
         }
         __syncwarp();
-        count = 0;
-        for (uint32_t w = lane; w < nw; w += 32) count += __popc(nxt[w]);
+        pos = b + 1;
+        uint32_t *cur = bm1, *nxt = bm0;
+        for (uint32_t w = lane; w < nw; w += 32) count += __popc(cur[w]);
         count = warp_sum_i32(count);
-        uint32_t *tmp = cur;
-        cur = nxt;
-        nxt = tmp;
-        ++pos;
-    }
-    if (count > 32) return -1;
-    // at most 32 members: one per lane
-    int32_t mine = 0;
-    for (uint32_t w = lane; w < nw; w += 32) mine += __popc(cur[w]);
-    int32_t before = mine;
+        // many members: bitmaps
+        while (count > kListMembers && pos < e) {
+            if ((count > kPollEveryStep || (pos - b) % kLatchPollSets == 0) &&
+                warp_latched_below(latch, index))
+                return -2;
+            const uint32_t c = __ldg(base + pos);
+            for (uint32_t w = lane; w < nw; w += 32) nxt[w] = 0u;
+            __syncwarp();
+            for (uint32_t w = lane; w < nw; w += 32) {
+                uint32_t bits = cur[w];
+                while (bits) {  // up to four lookups in flight per lane
+                    uint32_t s4[4];
+                    int k = 0;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int32_t y = __shfl_up_sync(GBFSM_FULL_MASK, before, d);
-        if ((int)lane >= d) before += y;
-    }
-    before -= mine;
-    for (uint32_t w = lane; w < nw; w += 32) {
-        uint32_t bits = cur[w];
-        while (bits) {
-            list[before++] = (w << 5) + (uint32_t)(__ffs(bits) - 1);
-            bits &= bits - 1u;
+                    for (int u = 0; u < 4; ++u) {
+                        if (bits) {
+                            s4[u] = (w << 5) + (uint32_t)(__ffs(bits) - 1);
+                            bits &= bits - 1u;
+                            k = u + 1;
+                        }
+                    }
+                    uint32_t t4[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (u < k) t4[u] = dfa_entry(T, s4[u], c) & ~ACC;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (u < k) atomicOr(nxt + (t4[u] >> 5), 1u << (t4[u] & 31u));
+                }
+            }
+            __syncwarp();
+            count = 0;
+            for (uint32_t w = lane; w < nw; w += 32) count += __popc(nxt[w]);
+            count = warp_sum_i32(count);
+            uint32_t *tmp = cur;
+            cur = nxt;
+            nxt = tmp;
+            ++pos;
         }
+        if (count > kListMembers) return -1;
+        // members to the list (bitmap bits in word order)
+        uint16_t *from = list, *to = list + kListMembers;
+        int32_t mine = 0;
+        for (uint32_t w = lane; w < nw; w += 32) mine += __popc(cur[w]);
+        int32_t before = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int32_t y = __shfl_up_sync(GBFSM_FULL_MASK, before, d);
+            if ((int)lane >= d) before += y;
+        }
+        before -= mine;
+        for (uint32_t w = lane; w < nw; w += 32) {
+            uint32_t bits = cur[w];
+            while (bits) {
+                from[before++] = (uint16_t)((w << 5) + (uint32_t)(__ffs(bits) - 1));
+                bits &= bits - 1u;
+            }
+            nxt[w] = 0u;  // the members seen in a step; all zero between steps
+        }
+        __syncwarp();
+        bytes.init(base + pos, e - pos);
+        while (count > 32 && pos < e) {
+            if (++polls % 4 == 0 && warp_latched_below(latch, index)) return -2;
+            // up to kMeetBytes bytes, then the members that met are dropped
+            const int k = (int)min((int64_t)kMeetBytes, e - pos);
+            uint32_t c[kMeetBytes];
+#pragma unroll
+            for (int j = 0; j < kMeetBytes; ++j) c[j] = j < k ? bytes.next() : 0u;
+            int32_t n_to = 0;
+            for (int32_t i0 = 0; i0 < count; i0 += 32 * 8) {  // eight lookups in flight
+                uint32_t t[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int32_t i = i0 + 32 * u + (int32_t)lane;
+                    t[u] = i < count ? from[i] : 0xffffffffu;
+                }
+#pragma unroll
+                for (int j = 0; j < kMeetBytes; ++j)
+                    if (j < k)
+#pragma unroll
+                        for (int u = 0; u < 8; ++u)
+                            if (t[u] != 0xffffffffu) t[u] = dfa_entry(T, t[u], c[j]) & ~ACC;
+                uint32_t seen[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    seen[u] = t[u] != 0xffffffffu ? atomicOr(nxt + (t[u] >> 5), 1u << (t[u] & 31u))
+                                                  : 0xffffffffu;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    if (i0 + 32 * u >= count) break;
+                    const bool fresh = !((seen[u] >> (t[u] & 31u)) & 1u);
+                    const uint32_t ball = __ballot_sync(GBFSM_FULL_MASK, fresh);
+                    if (fresh) to[n_to + __popc(ball & lanemask_lt())] = (uint16_t)t[u];
+                    n_to += __popc(ball);
+                }
+            }
+            __syncwarp();
+            for (int32_t i = (int32_t)lane; i < n_to; i += 32) nxt[to[i] >> 5] = 0u;
+            __syncwarp();
+            uint16_t *tmp = from;
+            from = to;
+            to = tmp;
+            count = n_to;
+            pos += k;
+        }
+        if (count > 32) return -1;
+        member = (int32_t)lane < count ? from[lane] : 0xffffffffu;
+        __syncwarp();
     }
-    __syncwarp();
-    bool active = (int32_t)lane < count;
-    uint32_t member = active ? list[lane] : 0xffffffffu;
-    __syncwarp();
-    uint32_t alive = __ballot_sync(GBFSM_FULL_MASK, active);
-    while (__popc(alive) > 1 && pos < e) {
-        if ((pos - b) % kLatchPollBytes == 0 && warp_latched_below(latch, index)) return -2;
-        const uint32_t c = __ldg(base + pos);
-        const uint32_t t = active ? (dfa_entry(T, member, c) & ~ACC) : 0xffffffffu;
-        const uint32_t same = __match_any_sync(GBFSM_FULL_MASK, t);
-        active = active && (uint32_t)(__ffs(same) - 1) == lane;
-        member = t;
-        alive = __ballot_sync(GBFSM_FULL_MASK, active);
-        ++pos;
+    // one member per lane (lanes without one hold 0xffffffff); of several that met, the
+    // first lane's stays
+    uint32_t alive = __ballot_sync(GBFSM_FULL_MASK, member != 0xffffffffu);
+    if (pos == b) bytes.init(base + pos, e - pos);  // (every state had a lane from the start)
+    while (__popc(alive) > want && pos < e) {
+        if (++polls % 64 == 0 && warp_latched_below(latch, index)) return -2;
+        const int k = (int)min((int64_t)kMeetBytes, e - pos);
+        if ((alive >> lane) & 1u) {
+#pragma unroll
+            for (int j = 0; j < kMeetBytes; ++j)
+                if (j < k) member = dfa_entry(T, member, bytes.next()) & ~ACC;
+        } else {
+            for (int j = 0; j < k; ++j) bytes.next();
+            member = 0xffffffffu;
+        }
+        __syncwarp();
+        const uint32_t same = __match_any_sync(GBFSM_FULL_MASK, member);
+        alive = __ballot_sync(GBFSM_FULL_MASK, ((alive >> lane) & 1u) &&
+                                                   (uint32_t)(__ffs(same) - 1) == lane);
+        pos += k;
     }
-    if (__popc(alive) != 1) return -1;
-    sigma = __shfl_sync(GBFSM_FULL_MASK, member, __ffs(alive) - 1);
+    count = __popc(alive);
+    if (count > want) return -1;
+    // members to lanes 0 .. count - 1
+    const uint32_t src = lane < (uint32_t)count ? select_bit(alive, lane) : 0u;
+    member = __shfl_sync(GBFSM_FULL_MASK, member, src);
     return pos;
 }
 
-// One lane: the overlap walk of a chunk ending at e, from its exact state s, into the next
-// chunk (record `next`, or NULL when e is the input's end): until the next chunk's
-// published collapse position has been passed, or it is known that the next chunk
-// stopped, or `cap` (at most the next chunk's end) is reached. Returns the overlap's
-// length; its first accept goes to ov_acc (-1 when none), the state at its end to
-// `s_end`, and `stopped` is set when a chunk below `index` latched the input meanwhile.
+// Collapse of chunk `index` of an input, spanning positions [b, e) of `base` (the input's
+// first byte): its entry position and states, to rec.
 template <typename Entry>
-__device__ int64_t dfa_overlap_walk(const Entry *T, uint32_t s, const uint8_t *base,
-                                    int64_t e, int64_t cap, const DfaChunkRecord *next,
-                                    const int32_t *latch, int32_t index, int64_t &ov_acc,
-                                    uint32_t &s_end, bool &stopped) {
-    constexpr uint32_t ACC = EntryTraits<Entry>::kAccept;
-    ov_acc = -1;
-    s_end = s;
-    if (cap <= e || !next) return 0;
-    ByteStream bs;
-    bs.init(base + e, cap - e);
-    int64_t q = e, target = cap;
-    while (q < target) {
-        if (latched_below(latch, index)) {
-            stopped = true;
-            break;
-        }
-        const int32_t np = __ldcv(&next->p);
-        if (np >= 0) target = min(target, max((int64_t)np, q));
-        else if (np == -2) target = q;  // -1 (never collapsed): on to the cap
-        const int64_t q1 = min(target, q + (int64_t)kLatchPollBytes);
-        for (; q < q1; ++q) {
-            const uint32_t x = dfa_entry(T, s, bs.next());
-            s = x & ~ACC;
-            if (x & ACC) {
-                ov_acc = q + 1;
-                s_end = s;
-                return ov_acc - e;
-            }
-        }
-    }
-    s_end = s;
-    return q - e;
-}
-
-// A DFA_CHUNK task: chunk `index` of an input spanning positions [b, e) of `base` (the
-// input's first byte), `len` bytes in all; the record goes to rec (the next chunk's, when
-// e < len, is rec_next, and that chunk ends at e_next). latch: the input's latch word, or
-// NULL.
-template <typename Entry>
-__device__ void dfa_chunk(const gbfsm_dfa_dev &d, int32_t overlap, const uint8_t *base,
-                          int64_t len, int64_t b, int64_t e, int64_t e_next, int index,
-                          uint32_t *bm0, uint32_t *bm1, uint32_t *list, DfaChunkRecord *rec,
-                          const DfaChunkRecord *rec_next, int32_t *latch) {
+__device__ void dfa_chunk_collapse(const gbfsm_dfa_dev &d, const uint8_t *base, int64_t b,
+                                   int64_t e, int index, uint32_t *bm0, uint32_t *bm1,
+                                   uint16_t *list, DfaChunkRecord *rec, int32_t *latch) {
     const Entry *T = static_cast<const Entry *>(d.table);
     const uint32_t lane = lane_id();
     int64_t p;
-    uint32_t s = 0;
-    int64_t acc = -1;
+    int32_t count = 1, acc = -1;
+    uint32_t member = (uint32_t)d.start_state;
     if (index == 0) {
-        p = 0;
-        s = (uint32_t)d.start_state;
-        if ((__ldg(d.accept_bits + (s >> 5)) >> (s & 31u)) & 1u) acc = 0;
+        // about as many steps as the other chunks' collapses take: an input that accepts
+        // early is then latched before most of its chunks' work is done
+        p = min(e, max((int64_t)1024, (int64_t)d.num_states / 4));
+        if (lane == 0) {
+            if ((__ldg(d.accept_bits + (member >> 5)) >> (member & 31u)) & 1u)
+                acc = 0;
+            else
+                member = dfa_walk_span(GlobalEntries<Entry>{T}, EntryTraits<Entry>::kAccept,
+                                       member, base, 0, (int32_t)p, acc);
+            if (latch && acc >= 0) atomicMin(latch, 0);
+        }
     } else {
-        if (lane == 0) __stcg(&rec->p, kPending);
-        p = dfa_collapse<Entry>(T, (uint32_t)d.num_states, base, b, e, bm0, bm1, list, s,
-                                latch, index);
-        if (lane == 0) __stcg(&rec->p, (int32_t)p);  // for the previous chunk's overlap
+        p = dfa_collapse<Entry>(T, (uint32_t)d.num_states, base, b, e, kEntries, bm0, bm1, list,
+                                member, count, latch, index);
     }
     if (lane == 0) {
-        int64_t ov_len = 0, ov_acc = -1;
-        uint32_t ov_state = 0;
-        bool stopped = false;
-        if (p >= 0 && acc < 0) {
-            s = dfa_span<Entry>(T, s, base, p, e, acc, latch, index, &stopped);
-            if (acc < 0 && !stopped) {
-                const int64_t cap =
-                    min(min(e + (int64_t)(overlap > 0 ? overlap : 0), e_next), len);
-                ov_len = dfa_overlap_walk<Entry>(T, s, base, e, cap, e < len ? rec_next : nullptr,
-                                                 latch, index, ov_acc, ov_state, stopped);
-                if (latch && ov_acc >= 0) atomicMin(latch, index + 1);
-            }
-        }
-        if (latch && acc >= 0) atomicMin(latch, index);
-        if (stopped) {  // the verdict lies in an earlier chunk: this record is never read
-            p = -2;
-            acc = ov_acc = -1;
-            ov_len = 0;
-        }
-        int4 *w = reinterpret_cast<int4 *>(rec);
-        w[0] = make_int4((int32_t)p, (int32_t)acc, (int32_t)s, (int32_t)ov_len);
-        w[1] = make_int4((int32_t)ov_acc, (int32_t)ov_state, 0, 0);
+        rec->p = (int32_t)p;
+        rec->at = p == -2 ? -1 : (int32_t)p;
+        rec->count = p >= 0 ? count : 0;
+        rec->done = p >= 0 ? (int32_t)p : 0;
+    }
+    if (lane < (uint32_t)kEntries) {
+        rec->entry[lane] = rec->exit[lane] = (uint16_t)member;
+        rec->acc[lane] = lane == 0 ? acc : -1;
     }
     __syncwarp();
 }
 
-// A DFA_FIXUP task (lane 0): the verdict of an input from its chunks' records (chunks[first
-// .. first + count), positions relative to the input's start `off`).
+// The whole warp, a chunk per half (kEntries lanes, one per entry state): walk the chunk of
+// record `rec` from its entry position to `target`; valid = false: this half has none.
+// latch: the input's latch word, or NULL. The halves stay in step, 256 bytes at a time, so
+// that their loads are in flight together.
+template <typename Entry>
+__device__ __forceinline__ void dfa_chunk_walk(bool valid, const Entry *table,
+                                               const uint8_t *base, int32_t target, int index,
+                                               DfaChunkRecord *rec, int32_t *latch) {
+    constexpr uint32_t ACC = EntryTraits<Entry>::kAccept;
+    const GlobalEntries<Entry> look{table};
+    const uint32_t lane = lane_id();
+    const int g = (int)(lane % kEntries);
+    const uint32_t half = ((1u << kEntries) - 1u) << (lane - (uint32_t)g);
+    int count = 0;
+    uint32_t s = 0;
+    int32_t acc = -1, q = 0;
+    if (valid) {
+        count = rec->count;
+        const int k = g < count ? g : 0;  // lanes past the entry states repeat the first's walk
+        s = rec->entry[k];
+        acc = rec->acc[k];
+        q = rec->p;
+    }
+    bool stopped = false, all = false;
+    for (;;) {
+        all = (__ballot_sync(GBFSM_FULL_MASK, acc >= 0) & half) == half;
+        bool more = valid && !all && !stopped && q < target;
+        const bool below = more && latched_below(latch, index);
+        const uint32_t stops = __ballot_sync(GBFSM_FULL_MASK, below);
+        stopped = stopped || (stops & half) != 0u;
+        more = more && !stopped;
+        if (!__any_sync(GBFSM_FULL_MASK, more)) break;
+        if (more) {
+            const int32_t to = target - q > kLatchPollBytes ? q + kLatchPollBytes : target;
+            if (acc < 0) s = dfa_walk_span(look, ACC, s, base, q, to, acc);
+            q = to;
+        }
+        __syncwarp();
+    }
+    if (!valid) return;
+    if (g < count) {
+        rec->exit[g] = (uint16_t)s;
+        rec->acc[g] = acc;
+    }
+    if (g == 0) {
+        if (all && latch) atomicMin(latch, index);
+        rec->done = q;
+        if (stopped) rec->p = -2;  // the verdict lies in an earlier chunk
+    }
+}
+
+// Where the walk of a chunk ending at e ends: at the next entry position of its input, or
+// the input's end, but at most `overlap` bytes past e.
+__device__ __forceinline__ int32_t dfa_walk_target(const gbfsm_chunk *chunks, int32_t n_chunks,
+                                                   const void *records, int32_t chunk,
+                                                   int64_t e, int64_t len, int32_t overlap) {
+    const int64_t cap = min(len, e + (int64_t)max(overlap, 0));
+    const int32_t input = chunks[chunk].input;
+    for (int32_t j = chunk + 1; j < n_chunks; ++j) {
+        if (chunks[j].input != input || chunks[j].index != chunks[j - 1].index + 1) break;
+        const int32_t at = dfa_record(records, j)->at;
+        if (at >= 0) return (int32_t)min(cap, (int64_t)at);
+    }
+    return (int32_t)cap;
+}
+
+// A DFA_FIXUP task (the whole warp): the verdict of an input from its chunks' records
+// (chunks first .. first + count).
 template <typename Entry>
 __device__ Verdict dfa_fixup(const gbfsm_dfa_dev &d, const uint8_t *base, int64_t len,
-                             const gbfsm_chunk *chunks, int64_t off, const void *records,
-                             int32_t first, int32_t count) {
-    const Entry *T = static_cast<const Entry *>(d.table);
-    const DfaChunkRecord r0 = *dfa_record(records, first);
-    if (r0.acc >= 0) return Verdict{1, r0.acc, r0.acc};
-    uint32_t s = (uint32_t)r0.end_state;
-    bool prev_ok = true;  // the previous chunk's walk and overlap are exact
-    int64_t prev_ov_len = r0.ov_len, prev_ov_acc = r0.ov_acc;
-    uint32_t prev_ov_state = (uint32_t)r0.ov_state;
-    for (int32_t k = 1; k < count; ++k) {
-        if (prev_ok && prev_ov_acc >= 0) return Verdict{1, (int32_t)prev_ov_acc, prev_ov_acc};
-        const gbfsm_chunk ch = chunks[first + k];
-        const int64_t b = ch.begin - off, e = ch.end - off;
-        const DfaChunkRecord r = *dfa_record(records, first + k);
-        int64_t acc;
-        if (r.p >= 0) {
-            if (!(prev_ok && r.p - b <= prev_ov_len)) {
-                dfa_span<Entry>(T, s, base, b, r.p, acc);  // the gap before the collapse
-                if (acc >= 0) return Verdict{1, (int32_t)acc, acc};
+                             const void *records, int32_t first, int32_t count) {
+    const GlobalEntries<Entry> look{static_cast<const Entry *>(d.table)};
+    constexpr uint32_t ACC = EntryTraits<Entry>::kAccept;
+    const uint32_t lane = lane_id();
+    uint32_t s = 0;
+    int32_t pos = 0, acc = -1;
+    bool known = false;
+    // the records do not depend on the state, so the next ones load while one is looked up
+    constexpr int kAhead = 8;
+    for (int32_t k0 = 0; k0 < count; k0 += kAhead) {
+        int32_t p[kAhead], n[kAhead], done[kAhead], a[kAhead];
+        uint32_t entry[kAhead], exit[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            p[u] = -1;
+            if (k0 + u < count) {
+                const DfaChunkRecord *r = dfa_record(records, first + k0 + u);
+                p[u] = r->p;
+                n[u] = r->count;
+                done[u] = r->done;
+                const uint32_t g = lane < (uint32_t)kEntries ? lane : 0u;
+                entry[u] = r->entry[g];
+                exit[u] = r->exit[g];
+                a[u] = r->acc[g];
             }
-            if (r.acc >= 0) return Verdict{1, r.acc, r.acc};
-            s = (uint32_t)r.end_state;
-            prev_ok = true;
-            prev_ov_len = r.ov_len;
-            prev_ov_acc = r.ov_acc;
-            prev_ov_state = (uint32_t)r.ov_state;
-        } else {
-            if (prev_ok && prev_ov_len == e - b) {
-                s = prev_ov_state;  // never collapsed, but the previous overlap covered it
-            } else {
-                s = dfa_span<Entry>(T, s, base, b, e, acc);  // never collapsed: walk it
-                if (acc >= 0) return Verdict{1, (int32_t)acc, acc};
-            }
-            prev_ok = false;
         }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            if (p[u] < 0) continue;
+            if (!known) {  // the first chunk's entry state is the true one
+                known = true;
+                s = __shfl_sync(GBFSM_FULL_MASK, entry[u], 0);
+            } else if (pos < p[u]) {
+                s = dfa_walk_span(look, ACC, s, base, pos, p[u], acc);  // every lane alike
+                if (acc >= 0) return Verdict{1, acc, acc};
+            } else if (pos > p[u]) {
+                continue;
+            }
+            const uint32_t hit = __ballot_sync(
+                GBFSM_FULL_MASK, (int32_t)lane < n[u] && lane < (uint32_t)kEntries && entry[u] == s);
+            pos = p[u];
+            if (hit == 0u) continue;
+            const int src = __ffs(hit) - 1;
+            const int32_t at = __shfl_sync(GBFSM_FULL_MASK, a[u], src);
+            if (at >= 0) return Verdict{1, at, at};
+            s = __shfl_sync(GBFSM_FULL_MASK, exit[u], src);
+            pos = done[u];
+        }
+    }
+    if (pos < len) {
+        s = dfa_walk_span(look, ACC, s, base, pos, (int32_t)len, acc);
+        if (acc >= 0) return Verdict{1, acc, acc};
     }
     return Verdict{0, 0, len};
 }

@@ -7,7 +7,9 @@
 // into the top bit of each entry, so one load per byte yields both the successor and
 // the latch test (the reference reads trans and then accept, dfa.cu:21-22).
 //
-// Input bytes are streamed with 16-byte loads (L1::no_allocate) one block ahead of use.
+// Input bytes are streamed with 16-byte loads (L1::no_allocate) one block ahead of use, four
+// at a time whatever their alignment, so that lanes on inputs of different alignments stay
+// together.
 #pragma once
 
 #include "common.cuh"
@@ -48,13 +50,51 @@ struct ArrayTable {
     }
 };
 
+// One lane: consume bytes [a, b) of `base` from state s. Returns the state at b, or at the
+// first accepting position q in (a, b], which goes to `acc` (-1 when none). Four lookups
+// are made before their accept flags are looked at, so that the chain of dependent loads
+// has no branch in it.
+template <typename Lookup>
+__device__ __forceinline__ uint32_t dfa_walk_span(const Lookup &look, uint32_t accept, uint32_t s,
+                                                  const uint8_t *base, int32_t a, int32_t b,
+                                                  int32_t &acc) {
+    acc = -1;
+    if (b <= a) return s;
+    WordStream words;
+    words.init(base + a, base + b);
+    for (int32_t q = a; q < b; q += 4) {
+        uint32_t w = words.next_word();
+        if (b - q >= 4) {
+            const uint32_t e0 = look(s, w & 0xffu);
+            const uint32_t e1 = look(e0 & ~accept, (w >> 8) & 0xffu);
+            const uint32_t e2 = look(e1 & ~accept, (w >> 16) & 0xffu);
+            const uint32_t e3 = look(e2 & ~accept, w >> 24);
+            if ((e0 | e1 | e2 | e3) & accept) {
+                const int t = (e0 & accept) ? 0 : (e1 & accept) ? 1 : (e2 & accept) ? 2 : 3;
+                acc = q + t + 1;
+                return (t == 0 ? e0 : t == 1 ? e1 : t == 2 ? e2 : e3) & ~accept;
+            }
+            s = e3;
+        } else {
+            for (int t = 0; t < b - q; ++t, w >>= 8) {
+                const uint32_t e = look(s, w & 0xffu);
+                s = e & ~accept;
+                if (e & accept) {
+                    acc = q + t + 1;
+                    return s;
+                }
+            }
+        }
+    }
+    return s;
+}
+
 // One input, one thread, table entries through `lookup(state, byte)`. Returns (flag,
 // len, examined) through references.
 template <typename Entry, typename Lookup>
 __device__ __forceinline__ void dfa_walk_with(const Lookup &table_at, const uint32_t *accept_bits,
                                               uint32_t start, const uint8_t *in, int64_t len,
                                               int32_t &flag, int32_t &mlen, int64_t &examined) {
-    constexpr uint32_t ACC = EntryTraits<Entry>::kAccept;
     flag = 0;
     mlen = 0;
     examined = len;
@@ -63,51 +103,16 @@ __device__ __forceinline__ void dfa_walk_with(const Lookup &table_at, const uint
         examined = 0;
         return;
     }
-    if (len <= 0) return;
-    const uint8_t *end = in + len;
-    const uint64_t addr = reinterpret_cast<uint64_t>(in);
-    const uint8_t *blk = reinterpret_cast<const uint8_t *>(addr & ~15ull);
-    int k = (int)(addr & 15ull);
-    uint4 cur4 = ld_stream16(blk);
-    uint4 nxt4 = make_uint4(0, 0, 0, 0);
-    if (blk + 16 < end) nxt4 = ld_stream16(blk + 16);
-    uint32_t cur = start;
-    int64_t pos = -(int64_t)k;  // position of byte 0 of the current block
-    for (;;) {
-        const int64_t remain = len - pos;  // bytes from the block start to the end
-        if (k == 0 && remain >= 16) {
-            // full block: 16 dependent lookups, latch tested per byte
-            const uint32_t w[4] = {cur4.x, cur4.y, cur4.z, cur4.w};
-#pragma unroll
-            for (int b = 0; b < 16; ++b) {
-                const uint32_t e = table_at(cur, (w[b >> 2] >> ((b & 3) * 8)) & 0xffu);
-                cur = e & ~ACC;
-                if (e & ACC) {
-                    flag = 1;
-                    mlen = (int32_t)(pos + b + 1);
-                    examined = pos + b + 1;
-                    return;
-                }
-            }
-        } else {
-            const int hi = remain < 16 ? (int)remain : 16;
-            for (int b = k; b < hi; ++b) {
-                const uint32_t e = table_at(cur, byte_of(cur4, b));
-                cur = e & ~ACC;
-                if (e & ACC) {
-                    flag = 1;
-                    mlen = (int32_t)(pos + b + 1);
-                    examined = pos + b + 1;
-                    return;
-                }
-            }
+    for (int64_t pos = 0; pos < len; pos += 1 << 30) {
+        int32_t acc;
+        start = dfa_walk_span(table_at, EntryTraits<Entry>::kAccept, start, in + pos, 0,
+                              (int32_t)min(len - pos, (int64_t)1 << 30), acc);
+        if (acc >= 0) {
+            flag = 1;
+            mlen = (int32_t)(pos + acc);
+            examined = pos + acc;
+            return;
         }
-        pos += 16;
-        k = 0;
-        if (pos >= len) return;
-        blk += 16;
-        cur4 = nxt4;
-        if (blk + 16 < end) nxt4 = ld_stream16(blk + 16);
     }
 }
 

@@ -91,7 +91,7 @@ gbfsm_status launch_dfa_chunks(const gbfsm_automaton *table, int32_t n_automata,
                                const int64_t *offsets, const int64_t *ends,
                                const gbfsm_chunk_io &chunk_io, int32_t max_states,
                                int32_t *flags, int32_t *lens, int32_t *examined,
-                               int32_t *latch, cudaStream_t stream);
+                               int32_t *latch, int32_t kind, cudaStream_t stream);
 size_t persistent_workspace_bytes(int32_t max_words, const gbfsm_plan &p);
 int32_t persistent_ctas_per_sm(int32_t max_words, const gbfsm_plan &p);
 gbfsm_status launch_nfa_layout(int32_t n, const int32_t *srp, const int32_t *stg,

@@ -5,10 +5,10 @@
 // plan_scan_kernel (one CTA of 1024 threads):
 //   1. classify every input by its automaton's class (whole-input NFA, warp-chunked NFA,
 //      lane-chunked NFA, DFA) and sum the bytes of the lane and warp classes;
-//   2. choose the chunk sizes: DFA chunks of an input are max(its DFA's shortest chunk,
-//      B / dfa_warps) bytes (B: the bytes of the DFA inputs holding two chunks of their
-//      own minimum), so that a batch of few long inputs gets short chunks and a large
-//      one a single wave of them; lane chunks get the smallest multiple of 64 bytes (at
+//   2. choose the chunk sizes: DFA chunks of an input are max(its DFA's shortest chunk, the
+//      batch's length) bytes, the latter balancing the cost of a chunk's collapse against
+//      its walk over the DFA inputs that hold two chunks of their own minimum, at most one
+//      wave of them; lane chunks get the smallest multiple of 64 bytes (at
 //      least min_chunk) whose chunks fill at most one wave of the lane launch (32 chunks
 //      per resident warp) -- found by an exponential then binary search, each probe a
 //      block-wide sum; warp chunks get a power of two giving about four chunks per
@@ -28,8 +28,8 @@
 //   inputs' chunk prefix counts, so that one long input's thousands of chunks do not
 //   fall to one warp; then the sentinel chunk of index 0 after the last, the LANES tasks
 //   (32 consecutive lane chunks each; every lane finds its own automaton) and the DFA
-//   groups (32 consecutive DFA inputs of the length-bucketed order; every lane finds its
-//   own DFA).
+//   groups (up to 32 consecutive DFA inputs of the length-bucketed order; every lane finds
+//   its own DFA).
 //
 // The reference has no counterpart: it launches one kernel per automaton and per call
 // with one thread or warp per whole input (src/gpufsm/backends/cuda/nfa.py:105-121).
@@ -43,6 +43,9 @@ constexpr int kPlanThreads = 1024;
 constexpr int kBuckets = 64;
 constexpr int kLaneGroup = 32;
 constexpr int64_t kMaxChunk = 1 << 20;
+// L2 gather rate x time of a dependent lookup / lookups of a collapse per byte of the
+// shortest chunk (150 G/s x 0.2 us / 50): see the DFA chunk length
+constexpr double kDfaBalance = 600.0;
 
 // per-input scratch (int32 arrays of n entries) and per-bucket tables
 struct PlanScratch {
@@ -181,6 +184,13 @@ __device__ __forceinline__ int64_t lane_size(const gbfsm_batch_plan_args &a, int
     return s > a.min_chunk ? s : a.min_chunk;
 }
 
+// DFA inputs per task: a lane each, but as few to a warp as the warps of the persistent
+// launch allow -- 32 walks on 32 tables take 0.5 us a byte in step, one alone 0.2 us.
+__device__ __forceinline__ int32_t dfa_group(const gbfsm_batch_plan_args &a, int32_t n_dfa) {
+    const int32_t warps = a.persist_warps > 0 ? a.persist_warps : 1;
+    return min((n_dfa + warps - 1) / warps, kLaneGroup);
+}
+
 __global__ void __launch_bounds__(kPlanThreads) plan_scan_kernel(gbfsm_batch_plan_args a,
                                                                  PlanScratch s) {
     __shared__ int64_t red[6 * 32 + 1];
@@ -195,7 +205,7 @@ __global__ void __launch_bounds__(kPlanThreads) plan_scan_kernel(gbfsm_batch_pla
     __syncthreads();
 
     // 1. classes and the bytes of the chunked classes
-    int64_t lane_bytes = 0, warp_bytes = 0, dfa_bytes = 0, dfa_long = 0;
+    int64_t lane_bytes = 0, warp_bytes = 0, dfa_bytes = 0, dfa_long = 0, dfa_work = 0;
     for (int32_t i = lo; i < hi; ++i) {
         const InputInfo r = input_info(a, i);
         s.cls[i] = r.cls;
@@ -207,25 +217,38 @@ __global__ void __launch_bounds__(kPlanThreads) plan_scan_kernel(gbfsm_batch_pla
             if (m > 0 && r.len >= 2 * m) {
                 dfa_bytes += r.len;
                 dfa_long += 1;
+                dfa_work += r.len * m;
             }
         }
     }
-    {  // the four totals in one block-wide pass
-        int64_t v4[4] = {lane_bytes, warp_bytes, dfa_bytes, dfa_long}, t4[4];
-        block_scan<4>(v4, t4, red);
-        lane_bytes = t4[0];
-        warp_bytes = t4[1];
-        dfa_bytes = t4[2];
-        dfa_long = t4[3];
+    {  // the totals in one block-wide pass
+        int64_t v5[5] = {lane_bytes, warp_bytes, dfa_bytes, dfa_long, dfa_work}, t5[5];
+        block_scan<5>(v5, t5, red);
+        lane_bytes = t5[0];
+        warp_bytes = t5[1];
+        dfa_bytes = t5[2];
+        dfa_long = t5[3];
+        dfa_work = t5[4];
     }
-    // the batch's DFA chunk length (before each DFA's minimum): rounding each input up to
-    // whole chunks adds at most one chunk per input, so B / (warps - inputs) keeps the
-    // chunks within one wave
+    // The batch's DFA chunk length (before each DFA's minimum m, a quarter of its states).
+    // A chunk costs the walk of its set of all states, about 50 m table lookups at the L2's
+    // gather rate R for the whole batch, and its own length L in dependent lookups of t
+    // each: the sum of B / L * 50 m / R and L t is least at L = sqrt(B m 50 / (R t)), with
+    // 50 / (R t) = 1 / kDfaBalance. And at most one wave of chunks: rounding each input up
+    // to whole chunks adds at most one per input, so B / (chunks at a time - inputs).
     int64_t dfa_target = 0;
+    bool dfa_split = false;
     if (a.dfa_warps > 0 && dfa_bytes > 0) {
         const int64_t w = a.dfa_warps > dfa_long ? a.dfa_warps - dfa_long : 1;
-        dfa_target = ((dfa_bytes + w - 1) / w + 63) / 64 * 64;
+        dfa_target = (dfa_bytes + w - 1) / w;
+        const int64_t balanced = (int64_t)sqrt((double)dfa_work / kDfaBalance);
+        if (balanced > dfa_target) dfa_target = balanced;
+        dfa_target = (dfa_target + 63) / 64 * 64;
         if (dfa_target > (int64_t)1 << 30) dfa_target = (int64_t)1 << 30;
+        // An input of less than two such chunks would be a single chain of up to 2 L
+        // lookups. Where there are few of them, each is cut into up to four chunks (none
+        // under its minimum), at most as many chunks again.
+        dfa_split = 3 * dfa_long * dfa_target <= dfa_bytes;
     }
 
     // 2. chunk sizes
@@ -294,7 +317,10 @@ __global__ void __launch_bounds__(kPlanThreads) plan_scan_kernel(gbfsm_batch_pla
         int64_t dfa_chunk = (c == GBFSM_PLAN_DFA && a.aut_dfa_chunk)
                                 ? (int64_t)a.aut_dfa_chunk[a.aut_ids ? a.aut_ids[i] : 0]
                                 : 0;
-        if (dfa_chunk > 0 && dfa_target > dfa_chunk) dfa_chunk = dfa_target;
+        if (dfa_chunk > 0) {
+            const int64_t l = dfa_split ? min(dfa_target, len / 4) : dfa_target;
+            if (l > dfa_chunk) dfa_chunk = l;
+        }
         if (c == GBFSM_PLAN_DFA && dfa_chunk > 0 && len >= 2 * dfa_chunk) {
             // a long DFA input: cut into chunks walked in parallel (DFA_CHUNK tasks)
             cnt = chunks_of(len, dfa_chunk);
@@ -360,12 +386,14 @@ __global__ void __launch_bounds__(kPlanThreads) plan_scan_kernel(gbfsm_batch_pla
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         if (lane == 0) {
-            int32_t d = 0, t = 0;
+            int32_t d = 0, t = 0, n_dfa = 0;
+            for (int b = 0; b < kBuckets; ++b) n_dfa += h_dfa[b];
+            const int32_t group = max(dfa_group(a, n_dfa), 1);
             for (int b = kBuckets - 1; b >= 0; --b) {  // DFA positions, longest bucket first
                 s.dbase[b] = d;
-                const int32_t g0 = (d + kLaneGroup - 1) / kLaneGroup;
+                const int32_t g0 = (d + group - 1) / group;
                 d += h_dfa[b];
-                h_grp[b] = (d + kLaneGroup - 1) / kLaneGroup - g0;
+                h_grp[b] = (d + group - 1) / group - g0;
             }
             s.dbase[kBuckets] = d;
             for (int b = kBuckets - 1; b >= 0; --b) {  // persistent slots, longest first
@@ -526,15 +554,16 @@ __global__ void __launch_bounds__(256) plan_fill_kernel(gbfsm_batch_plan_args a,
         const int32_t first = (int32_t)t * kLaneGroup;
         tl[t] = gbfsm_task{-1, first, min(kLaneGroup, n_lane - first), GBFSM_TASK_LANES};
     }
-    // DFA groups: 32 consecutive positions of the bucketed DFA order
-    const int32_t n_groups = (n_dfa + kLaneGroup - 1) / kLaneGroup;
+    // DFA groups: consecutive positions of the bucketed DFA order
+    const int32_t group = max(dfa_group(a, n_dfa), 1);
+    const int32_t n_groups = (n_dfa + group - 1) / group;
     for (int64_t g = tid; g < n_groups; g += nthreads) {
-        const int32_t p = (int32_t)g * kLaneGroup;
+        const int32_t p = (int32_t)g * group;
         int b = kBuckets - 1;
         while (b > 0 && p >= s.dbase[b - 1]) --b;  // bucket b holds [dbase[b], dbase[b-1])
-        const int32_t g_first = (s.dbase[b] + kLaneGroup - 1) / kLaneGroup;
+        const int32_t g_first = (s.dbase[b] + group - 1) / group;
         tp[s.tdfa[b] + ((int32_t)g - g_first)] =
-            gbfsm_task{-1, n_whole + p, min(kLaneGroup, n_dfa - p), GBFSM_TASK_DFA_GROUP};
+            gbfsm_task{-1, n_whole + p, min(group, n_dfa - p), GBFSM_TASK_DFA_GROUP};
     }
 }
 

@@ -30,6 +30,7 @@ backends/cuda/nfa.py:105-121).
 from __future__ import annotations
 
 import ctypes
+import math
 import time
 from dataclasses import dataclass, field
 
@@ -52,27 +53,26 @@ MIN_CHUNK = 256      # shortest speculative chunk (bytes)
 MIN_CHUNK_SMALL_STARTS = 64
 LANE_GROUP = 32      # chunks per LANES task (one per lane)
 # an automaton's chunks run one per lane when its two-byte supersets are this small on
-# average: a lane starts from the superset when it has at most native.LANE_CAPACITY
-# states, else from the superset two bytes earlier stepped over the two bytes (up to 64
-# states streamed once); sets that outgrow the lane spill to warps
+# average: a lane starts from the superset when it fits the lane (8 states over a slot
+# table, else native.LANE_CAPACITY), else from the superset two bytes earlier stepped over
+# the two bytes (up to 64 states streamed once); sets that outgrow the lane spill to warps
 LANE_PAIR_MEAN = 32.0
-# resident warps per SM of the lane launch when the device is not asked (128-thread
-# CTAs, 8 per SM: csrc/lanes.cu)
+# resident warps per SM of the lane launch when the device is not asked (64 registers a
+# thread: csrc/lanes.cu)
 LANE_WARPS_PER_SM = 32
 # DFA chunking (csrc/dfa_chunks.cu): the largest DFA whose inputs are chunked (2-byte
-# table entries), and the shortest DFA chunk: at least DFA_CHUNK_MIN bytes and
-# DFA_CHUNK_PER_STATE bytes per state. A random DFA's set of all states collapses after
-# about 2n bytes, with a tail of about e^(-t/n) beyond; at 8n a chunk rarely ends before
-# it collapses (at 2n about half do, and their fix-up turns serial). The planner
-# lengthens the chunks of a batch with many long DFA inputs to one wave of the chunk
-# launch.
+# table entries), and the shortest DFA chunk: at least DFA_CHUNK_MIN bytes and a byte per
+# DFA_CHUNK_STATES states. A chunk follows the set of all states until it has 16 members,
+# which takes a random DFA about n / 8 bytes; twice that leaves room for slower ones (a
+# chunk that ends before is walked through by the one before it). The planner lengthens the
+# chunks of larger batches.
 DFA_CHUNK_MAX_STATES = 32768
-DFA_CHUNK_MIN = 16 << 10
-DFA_CHUNK_FLOOR = 4096  # the shortest DFA chunk a caller may ask for
-DFA_CHUNK_PER_STATE = 8
-# the most a DFA chunk's exact walk continues into the next chunk, as a share of the
-# shortest chunk; 1 or more: no limit but the next chunk's end (the walk stops at that
-# chunk's collapse, or covers it whole when it never collapses)
+DFA_CHUNK_MIN = 1024
+DFA_CHUNK_FLOOR = 1024  # the shortest DFA chunk a caller may ask for
+DFA_CHUNK_STATES = 4
+DFA_CHUNK_BALANCE = 600.0  # kDfaBalance (csrc/plan.cu)
+# the most a DFA chunk's walk continues past its end, as a share of the shortest chunk; 1 or
+# more: no limit but the next entry position
 DFA_OVERLAP_CHUNKS = 1.0
 # a host batch the device gathers in place (staging.py) of at least PIPELINE_MIN_BYTES is
 # gathered in PIPELINE_PARTS slices of contiguous inputs, each slice's lane tasks starting
@@ -88,11 +88,11 @@ PIPELINE_LANE_WAVES = 2
 def dfa_chunk_length(num_states: int) -> int:
     """Shortest chunk for the long inputs of a DFA of ``num_states`` states (a multiple of
     64 bytes); an input is chunked when it holds two chunks."""
-    return -(-max(DFA_CHUNK_MIN, DFA_CHUNK_PER_STATE * int(num_states)) // 64) * 64
+    return -(-max(DFA_CHUNK_MIN, int(num_states) // DFA_CHUNK_STATES) // 64) * 64
 
 
 def dfa_overlap_bytes(chunk_length: int) -> int:
-    """Most bytes a DFA chunk's exact walk continues into the next chunk."""
+    """Most bytes a DFA chunk's walk continues past its end."""
     if DFA_OVERLAP_CHUNKS >= 1.0:
         return 1 << 30
     return int(DFA_OVERLAP_CHUNKS * int(chunk_length))
@@ -260,12 +260,17 @@ class DevicePlan:
     @staticmethod
     def dfa_caps(engine: PersistentEngine, n: int, total_bytes: int) -> tuple[int, int]:
         """Capacities for DFA chunks and DFA fix-ups: an input is chunked when it holds
-        at least two chunks of its DFA, so it has at most 1.5 x its bytes / chunk chunks."""
+        at least two chunks of its DFA, so it has at most 1.5 x its bytes / chunk chunks
+        (chunk: the shortest, or the planner's length for this many bytes, with at most as
+        many chunks again for inputs shorter than that)."""
         if engine.aut_dfa_chunk is None:
             return 0, 0
         c = engine.min_dfa_chunk
-        return (3 * int(total_bytes) // (2 * c) + 2,
-                min(int(n), int(total_bytes) // (2 * c)) + 1)
+        fixups = min(int(n), int(total_bytes) // (2 * c)) + 1
+        if engine.dfa_warps > 0:
+            length = max(c, int(math.sqrt(int(total_bytes) * c / DFA_CHUNK_BALANCE)))
+            return 3 * int(total_bytes) // length + 2, fixups
+        return 3 * int(total_bytes) // (2 * c) + 2, fixups
 
     @staticmethod
     def device_bytes(engine: PersistentEngine, n_inputs: int, total_bytes: int) -> int:
@@ -349,7 +354,7 @@ class DevicePlan:
 
     def launch(self, data_ptr: int, d_off, d_ends, d_flags, d_lens, d_examined, stream,
                workspace=None, phases: dict | None = None, lane_slices=None) -> int:
-        """Enqueue the launches of a planned batch (four, six when the pool chunks long DFA
+        """Enqueue the launches of a planned batch (four, seven when the pool chunks long DFA
         inputs); returns their number.
         ``lane_slices``: ``[(side stream, ready event)]`` per slice (pipelined ingest);
         slice k's lane tasks run on its side stream once its event has fired."""
@@ -396,22 +401,22 @@ class DevicePlan:
             mark("lanes")
             launches += 1
 
-        def dfa_chunks(name, tasks_ptr, max_tasks, count_word):
+        def dfa_chunks(name, tasks_ptr, max_tasks, count_word, kind):
             mark(name)
-            st = lib.gbfsm_dfa_chunks_run(
+            st = lib.gbfsm_dfa_chunks_run_kind(
                 table, n_aut, tasks_ptr, int(max_tasks), self._hdr(count_word), data_ptr,
                 d_off.data_ptr(), d_ends.data_ptr() if d_ends is not None else None,
                 ctypes.byref(io), eng.dfa_max_states, d_flags.data_ptr(), d_lens.data_ptr(),
                 d_examined.data_ptr() if d_examined is not None else None,
-                self.dfa_latch.data_ptr(), stream.cuda_stream)
-            native.check(st, "gbfsm_dfa_chunks_run")
+                self.dfa_latch.data_ptr(), kind, stream.cuda_stream)
+            native.check(st, "gbfsm_dfa_chunks_run_kind")
             mark(name)
 
         chunked_dfa = eng.aut_dfa_chunk is not None and self.cap_dfa_chunks > 0
         if chunked_dfa:
             dfa_chunks("dfa_chunks", self.tasks_dfa_chunk, self.cap_dfa_chunks,
-                       native.PLAN_DFA_CHUNKS)
-            launches += 1
+                       native.PLAN_DFA_CHUNKS, native.TASK_DFA_CHUNK)
+            launches += 2
 
         def persist(name, tasks_ptr, max_tasks, count_word):
             mark(name)
@@ -431,7 +436,7 @@ class DevicePlan:
         persist("fixup", self.tasks_fixup, self.cap_fixup, native.PLAN_FIXUP_TASKS)
         if chunked_dfa:
             dfa_chunks("dfa_fixup", self.tasks_dfa_fixup, self.cap_dfa_fixup,
-                       native.PLAN_DFA_FIXUPS)
+                       native.PLAN_DFA_FIXUPS, native.TASK_DFA_FIXUP)
             launches += 1
         return launches + 3
 
@@ -499,11 +504,7 @@ class PersistentEngine:
             self.ws_bytes = int(lib.gbfsm_persistent_workspace_bytes(self.max_words,
                                                                      ctypes.byref(self.plan)))
             self.workspace = torch.zeros(self.ws_bytes, dtype=torch.uint8, device=self.device)
-            # long DFA inputs are cut into chunks walked in parallel (DFA_CHUNK tasks): a
-            # chunk of an n-state DFA spans at least max(16 KiB, 8n) bytes, and its exact
-            # walk continues into the next chunk until it passes that chunk's collapse
-            # (about 2n bytes in for a random DFA), or over all of it when it never
-            # collapses
+            # long DFA inputs are cut into chunks walked in parallel (DFA_CHUNK tasks)
             dfa_chunk = [0] * len(self.automata)
             if chunk_bytes is not None and dfa_chunk_bytes != 0:
                 for i, (d, k) in enumerate(zip(self.dev, self.kinds)):

@@ -245,6 +245,9 @@ SIGNATURES: dict[str, tuple] = {
     "gbfsm_dfa_chunks_warps_per_sm": (_i32, [_i32]),
     "gbfsm_dfa_chunks_run": (ctypes.c_int, [_vp, _i32, _vp, _i32, _vp, _vp, _vp, _vp,
                                             _P(ChunkIO), _i32, _vp, _vp, _vp, _vp, _vp]),
+    "gbfsm_dfa_chunks_run_kind": (ctypes.c_int, [_vp, _i32, _vp, _i32, _vp, _vp, _vp, _vp,
+                                                 _P(ChunkIO), _i32, _vp, _vp, _vp, _vp, _i32,
+                                                 _vp]),
 }
 
 ABI_VERSION = 4

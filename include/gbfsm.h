@@ -278,8 +278,8 @@ typedef struct gbfsm_automaton {
     int32_t kind;          /* 0 = NFA, 1 = DFA */
     int32_t technique;     /* NFA: GBFSM_TECH_WARP or GBFSM_TECH_COMPACT */
     int32_t list_capacity; /* NFA compact list capacity (<= the launch's capacity) */
-    int32_t dfa_overlap;   /* DFA: the most bytes a DFA_CHUNK task's exact walk continues
-                              past its chunk's end, never past the next chunk's end (0 =
+    int32_t dfa_overlap;   /* DFA: the most bytes a DFA_CHUNK task's walk continues past its
+                              chunk's end, towards the next chunk's entry position (0 =
                               none: every chunk then links by a serial walk) */
     gbfsm_nfa_dev nfa;     /* valid when kind == 0 */
     gbfsm_dfa_dev dfa;     /* valid when kind == 1 */
@@ -312,9 +312,9 @@ typedef struct gbfsm_task {
                                   DFA walk per lane, each on its input's own DFA
                                   (gbfsm_chunk_io.aut_ids); automaton is -1 */
 #define GBFSM_TASK_DFA_CHUNK 5 /* chunk `first` (count 1) of a long input of DFA `automaton`,
-                                  walked by a warp from the set of all states until it
-                                  collapses to one; its record goes to the chunk records
-                                  (gbfsm_dfa_chunks_run) */
+                                  walked from the set of all states until it collapses to a
+                                  few, then from each of those; its record goes to the chunk
+                                  records (gbfsm_dfa_chunks_run) */
 #define GBFSM_TASK_DFA_FIXUP 6 /* input whose DFA chunks are chunks[first .. first + count):
                                   its exact verdict from their records, gaps walked
                                   serially (gbfsm_dfa_chunks_run) */
@@ -509,13 +509,13 @@ typedef struct gbfsm_batch_plan_args {
     int32_t lane_warps;       /* resident warps of the lane launch (SMs x
                                  gbfsm_lanes_warps_per_sm) */
     int32_t persist_warps;    /* resident warps of the persistent launch */
-    int32_t dfa_warps;        /* resident warps of the DFA chunk launch (SMs x
+    int32_t dfa_warps;        /* chunks that the DFA chunk launch walks at a time (SMs x
                                  gbfsm_dfa_chunks_warps_per_sm), or 0. An input of DFA a is
-                                 cut into chunks of max(aut_dfa_chunk[a], B / dfa_warps)
-                                 bytes, B the bytes of the batch's DFA inputs that hold two
-                                 chunks of their own minimum, when it holds two of them:
-                                 short chunks when few long inputs leave warps idle, one
-                                 wave of chunks otherwise */
+                                 cut into chunks of max(aut_dfa_chunk[a], L) bytes when it
+                                 holds two of them; L balances the cost of a chunk's
+                                 collapse (its minimum's share) against its walk over the
+                                 batch's DFA inputs that hold two chunks of their own
+                                 minimum, at most dfa_warps chunks (csrc/plan.cu) */
     int32_t min_chunk;        /* shortest chunk (bytes) */
     int32_t fixed_chunk;      /* > 0: every chunk size; 0: chosen; < 0: never chunk */
     int32_t n_slices;         /* 0 or 1: one lane range; else inputs cut into slices at
@@ -550,15 +550,14 @@ size_t gbfsm_batch_plan_scratch_bytes(int32_t n_inputs);
  * device-side failures (capacity, automaton ids) are reported in the header's status. */
 gbfsm_status gbfsm_batch_plan(const gbfsm_batch_plan_args *args, void *stream);
 
-/* Resident warps per SM of gbfsm_dfa_chunks_run for DFAs of up to max_states states (its
- * shared scratch grows with them); 0 when the query fails. */
+/* Chunks per SM that gbfsm_dfa_chunks_run walks at a time for DFAs of up to max_states
+ * states; 0 when it cannot run. */
 int32_t gbfsm_dfa_chunks_warps_per_sm(int32_t max_states);
 
 /* Run DFA_CHUNK or DFA_FIXUP tasks (others are skipped): min(*task_count, max_tasks)
  * tasks of `tasks` when task_count is non-NULL, else max_tasks. A step runs the DFA_CHUNK
  * tasks of a batch first, then its DFA_FIXUP tasks in a later launch on the same stream;
- * both read chunk_io->chunks and share chunk_io->records (the first 32 bytes of each
- * chunk's record). max_states: the most states of any DFA the tasks name (1..32768; each
+ * both read chunk_io->chunks and share chunk_io->records. max_states: the most states of any DFA the tasks name (1..32768; each
  * warp holds two bitmaps of that many bits in shared memory). A DFA_FIXUP task writes its
  * input's flags / lens (and examined) entries. Input i is data[offsets[i] .. ends[i]) when
  * `ends` is non-NULL, else data[offsets[i] .. offsets[i + 1]). latch (device [n_inputs] or
@@ -576,6 +575,16 @@ gbfsm_status gbfsm_dfa_chunks_run(const gbfsm_automaton *table, int32_t n_automa
                                   const gbfsm_chunk_io *chunk_io, int32_t max_states,
                                   int32_t *flags, int32_t *lens, int32_t *examined,
                                   int32_t *latch, void *stream);
+
+/* gbfsm_dfa_chunks_run for a task list of one kind (GBFSM_TASK_DFA_CHUNK or
+ * GBFSM_TASK_DFA_FIXUP; 0: either), without the launches that the other kind needs. */
+gbfsm_status gbfsm_dfa_chunks_run_kind(const gbfsm_automaton *table, int32_t n_automata,
+                                       const gbfsm_task *tasks, int32_t max_tasks,
+                                       const int32_t *task_count, const uint8_t *data,
+                                       const int64_t *offsets, const int64_t *ends,
+                                       const gbfsm_chunk_io *chunk_io, int32_t max_states,
+                                       int32_t *flags, int32_t *lens, int32_t *examined,
+                                       int32_t *latch, int32_t kind, void *stream);
 
 /* Occupancy query for persistent launches: CTAs of `plan` resident per SM. */
 int32_t gbfsm_persistent_ctas_per_sm(int32_t max_words, const gbfsm_plan *plan);

@@ -1,0 +1,72 @@
+"""Chunked DFA walks by entry states (csrc/dfa_chunks.cuh) against the oracle (GPU), where
+the collapse changes form: DFAs of as many states as a chunk has entry states, a warp has
+lanes or the member list has places, and one more; sets that stay too large; accepts so
+frequent that some entry states' walks accept and others do not (a warp walks two chunks,
+which stop at different bytes)."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from abstraction_regret_gb300.automata import DFA, random_dfa
+from abstraction_regret_gb300.engine import PersistentEngine
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(dfa, inputs, **kw):
+    eng = PersistentEngine([dfa], **kw)
+    f, l, e, _, _ = eng.run_requests([0] * len(inputs), inputs, with_examined=True)
+    data, off = O.flatten(inputs)
+    of, ol, oe = O.dfa_batch(dfa, data, off)
+    assert np.array_equal(f, of) and np.array_equal(l, ol) and np.array_equal(e, oe)
+    return of
+
+
+@pytest.mark.parametrize("states", [1, 2, 16, 17, 32, 33, 1024, 1025, 1500, 4097])
+@pytest.mark.parametrize("accept", [0.0, 0.0002, 0.002])
+def test_random_dfas_of_every_form(states, accept):
+    dfa = random_dfa(states, accept_prob=accept, seed=states)
+    if accept and states > 16:  # at least one accepting state, never the start
+        acc = dfa.accept.copy()
+        acc[0], acc[-1] = False, True
+        dfa = DFA(num_states=states, start_state=0, accept=acc, trans=dfa.trans)
+    rng = np.random.default_rng(states)
+    lengths = np.concatenate([rng.integers(0, 2048, 20), rng.integers(2048, 40000, 40),
+                              [1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097]])
+    inputs = [rng.integers(0, 256, int(n), dtype=np.uint8).tobytes() for n in lengths]
+    _check(dfa, inputs)
+
+
+@pytest.mark.parametrize("group", [8, 16, 17, 40])
+def test_sets_that_stop_shrinking(group):
+    """States of a ``group`` are permuted by every byte: the set of all states shrinks to
+    the group and no further (up to 16: entry states that never meet; above: no entry
+    states, every chunk walked through by the first one)."""
+    rng = np.random.default_rng(group)
+    n = 200
+    trans = rng.integers(0, group, size=(n, 256))
+    for c in range(256):
+        trans[:group, c] = rng.permutation(group)
+    trans[0, 7] = n - 1  # a rare way to the accepting state
+    accept = np.arange(n) == n - 1
+    dfa = DFA(num_states=n, start_state=1, accept=accept, trans=trans.reshape(-1).astype(np.int32))
+    inputs = []
+    for k in range(12):
+        x = rng.integers(8, 256, 9000 + 777 * k, dtype=np.uint8)
+        if k % 3:
+            x[rng.integers(0, x.size, k)] = 7
+        inputs.append(x.tobytes())
+    flags = _check(dfa, inputs)
+    assert 0 < int(flags.sum()) < len(inputs)
+
+
+def test_few_and_many_short_inputs():
+    """DFA groups of one input and of several (more inputs than resident warps)."""
+    dfa = random_dfa(300, accept_prob=0.004, seed=5)
+    rng = np.random.default_rng(6)
+    for n in (3, 6000):
+        _check(dfa, [rng.integers(0, 256, int(k), dtype=np.uint8).tobytes()
+                     for k in rng.integers(0, 400, n)])
