@@ -67,6 +67,7 @@ struct ChunkIO {
     const int32_t *task_count;
     int32_t n_chunks;
     const int32_t *aut_ids;  // per-input automaton (NULL: all 0)
+    int32_t sym_fixups;      // FIXUP tasks of automata with symbol lists have their own launch
 };
 
 __device__ __forceinline__ uint32_t byte_at(const uint8_t *p) { return __ldg(p); }
@@ -169,11 +170,12 @@ __device__ __forceinline__ void write_overlap(ChunkRecord *rec, int32_t ov_len, 
 }
 
 // b, e, ov_end: input-relative bounds of the chunk and of its overlap run.
+template <typename Stepper>
 __device__ inline void run_chunk(const gbfsm_nfa_dev &nfa, const Rows &R, WarpScratch S,
                                  const uint8_t *base, int64_t b, int64_t e, int64_t ov_end,
                                  int index, ChunkRecord *rec) {
     const uint32_t lane = lane_id();
-    WarpNfa<false> w(nfa, R, S);
+    Stepper w(nfa, R, S);
     int32_t counts[kCheckpoints], acc_after[kCheckpoints];
 #pragma unroll
     for (int c = 0; c < kCheckpoints; ++c) {
@@ -190,9 +192,7 @@ __device__ inline void run_chunk(const gbfsm_nfa_dev &nfa, const Rows &R, WarpSc
             stopped = true;
         }
     } else {
-        const uint32_t c0 = byte_at(base + b - 2);
-        ev = w.init_records(nfa.first_edges, __ldg(nfa.first_row + c0),
-                            __ldg(nfa.first_row + c0 + 1));
+        ev = w.init_after(byte_at(base + b - 2));
         if (ev != kDead) ev = w.step(byte_at(base + b - 1));
         if (ev == kDead) {
             dead_at = (int32_t)b;
@@ -200,12 +200,13 @@ __device__ inline void run_chunk(const gbfsm_nfa_dev &nfa, const Rows &R, WarpSc
         }
     }
     const int64_t len = e - b;
-    ByteStream bytes;
+    BytesAhead bytes;
     bytes.init(base + b, stopped ? 0 : len);
     int64_t j = 0;
     while (!stopped && j < len) {
-        ev = w.step(bytes.next());
         ++j;
+        const uint32_t sym = bytes.advance();
+        ev = w.step(sym, bytes.next, bytes.next2);
         const int32_t pos = (int32_t)(b + j);
         if (ev == kDead) {
             dead_at = pos;
@@ -220,7 +221,7 @@ __device__ inline void run_chunk(const gbfsm_nfa_dev &nfa, const Rows &R, WarpSc
             }
         }
         const int c = checkpoint_of(j);
-        if (c >= 0 && ev != kDead) counts[c] = w.m;
+        if (c >= 0 && ev != kDead) counts[c] = w.count();
     }
     int32_t end_count = -1;
     int32_t ov_len = 0, ov_event = 0, ov_counts[kCheckpoints];
@@ -241,7 +242,7 @@ __device__ inline void run_chunk(const gbfsm_nfa_dev &nfa, const Rows &R, WarpSc
                 break;
             }
             const int c = checkpoint_of(t);
-            if (c >= 0) ov_counts[c] = w.m;
+            if (c >= 0) ov_counts[c] = w.count();
         }
     }
     if (lane == 0) {
@@ -798,17 +799,23 @@ __device__ inline Verdict serial_fixup(WarpNfa<false> &w, const uint8_t *base, i
     return v;
 }
 
-__device__ inline Verdict run_fixup(const gbfsm_nfa_dev &nfa, const Rows &R, WarpScratch S,
-                                    const uint8_t *base, int64_t len, const ChunkRecord *recs,
-                                    int first, int count) {
+// One warp: the link scan over an input's chunk records. True when it decides the input (v);
+// else last_rec is the last chunk whose recorded end set is exact (-1: not even the first's).
+__device__ inline bool scan_links(const ChunkRecord *recs, int first, int count, Verdict &v,
+                                  int &last_rec) {
     const uint32_t lane = lane_id();
     const ChunkRecord &r0 = recs[first];
-    if (r0.acc_after[0] >= 0) return decided(1, r0.acc_after[0]);
-    if (r0.dead_at >= 0) return decided(0, r0.dead_at);
-    // scan: 32 chunks per round, one per lane; stop at the first that is not linked
-    int last_rec = r0.end_count >= 0 ? 0 : -1;  // last chunk with an exact recorded end set
-    int brk = -1;
-    for (int k0 = 1; k0 < count && brk < 0; k0 += 32) {
+    if (r0.acc_after[0] >= 0) {
+        v = decided(1, r0.acc_after[0]);
+        return true;
+    }
+    if (r0.dead_at >= 0) {
+        v = decided(0, r0.dead_at);
+        return true;
+    }
+    // 32 chunks per round, one per lane; stop at the first that is not linked
+    last_rec = r0.end_count >= 0 ? 0 : -1;
+    for (int k0 = 1; k0 < count; k0 += 32) {
         const int k = k0 + (int)lane;
         int status = kLink;
         int32_t flag = 0;
@@ -828,11 +835,21 @@ __device__ inline Verdict run_fixup(const gbfsm_nfa_dev &nfa, const Rows &R, War
             status = __shfl_sync(GBFSM_FULL_MASK, status, src);
             flag = __shfl_sync(GBFSM_FULL_MASK, flag, src);
             pos = __shfl_sync(GBFSM_FULL_MASK, pos, src);
-            if (status == kDecide) return decided(flag, pos);
-            brk = k0 + src;
+            if (status == kDecide) v = decided(flag, pos);
+            return status == kDecide;
         }
     }
-    if (brk < 0) return Verdict{0, 0, len};  // every chunk linked, no event: no accept
+    return true;  // every chunk linked, no event: no accept (v as the caller set it)
+}
+
+// The fix-up of one input by a warp (inputs of automata with symbol lists have a CTA:
+// sym_fixup.cu).
+__device__ inline Verdict run_fixup(const gbfsm_nfa_dev &nfa, const Rows &R, WarpScratch S,
+                                    const uint8_t *base, int64_t len, const ChunkRecord *recs,
+                                    int first, int count) {
+    Verdict v{0, 0, len};
+    int last_rec = -1;
+    if (scan_links(recs, first, count, v, last_rec)) return v;
     // fall back: serial from the chunk after the last exact recorded end set
     WarpNfa<false> w(nfa, R, S);
     int start;
@@ -846,7 +863,7 @@ __device__ inline Verdict run_fixup(const gbfsm_nfa_dev &nfa, const Rows &R, War
         for (int64_t p = 0; p < e0; ++p) w.step(byte_at(base + p));
         start = 1;
     }
-    const Verdict v = serial_fixup(w, base, len, recs, first, start, count);
+    v = serial_fixup(w, base, len, recs, first, start, count);
     w.cleanup();
     return v;
 }

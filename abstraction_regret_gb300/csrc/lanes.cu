@@ -227,7 +227,7 @@ gbfsm_status launch_lanes(const gbfsm_automaton *table, int32_t n_automata,
     const int32_t share = chunk_io.lane_share > 1 ? chunk_io.lane_share : 1;
     ChunkIO io{chunk_io.chunks, static_cast<ChunkRecord *>(chunk_io.records),
                chunk_io.overflow_tasks, chunk_io.overflow_count, nullptr, chunk_io.n_chunks,
-               chunk_io.aut_ids};
+               chunk_io.aut_ids, 0};
     if (chunk_io.lane_stage != 0 && n_automata == 1) {
         const bool narrow = chunk_io.lane_stage == GBFSM_LANE_STAGE_NARROW;
         if (chunk_io.lane_stage_bytes < 0 || chunk_io.lane_stage_bytes > lanes_stage_limit())

@@ -494,8 +494,18 @@ struct WarpNfa {
         return (info & GBFSM_EDGE_ACCEPT) ? kAccept : kAlive;
     }
 
-    __device__ __forceinline__ int step(uint32_t sym) {
+    // (the bytes after, `next` and `next2`, are for steppers that load ahead)
+    __device__ __forceinline__ int step(uint32_t sym, int next = -1, int next2 = -1) {
+        (void)next;
+        (void)next2;
         return mode == kReg ? step_reg(sym) : step_general(sym);
+    }
+
+    __device__ __forceinline__ int count() const { return m; }
+
+    // The superset of a chunk start: whatever the set was before byte c.
+    __device__ __forceinline__ int init_after(uint32_t c) {
+        return init_records(A.first_edges, __ldg(A.first_row + c), __ldg(A.first_row + c + 1));
     }
 
     // Start from the set of records recs[rb .. re) (distinct states), closed under epsilon
@@ -568,12 +578,34 @@ struct WarpNfa {
     }
 };
 
-// Simulate one input with a whole warp. All lanes call it with identical arguments and
-// all receive the verdict. `R` may point at shared-memory copies of the edge rows.
-template <bool kStaged>
-__device__ Verdict simulate_warp(const gbfsm_nfa_dev &A, const Rows &R, const uint8_t *in,
-                                 int64_t len, WarpScratch S) {
-    WarpNfa<kStaged> w(A, R, S);
+// A byte stream with the two bytes after the current one (-1 past the end).
+struct BytesAhead {
+    ByteStream bytes;
+    int64_t left;  // bytes not yet taken from the stream
+    int now, next, next2;
+
+    __device__ __forceinline__ int take() { return left > 0 ? (--left, (int)bytes.next()) : -1; }
+
+    __device__ __forceinline__ void init(const uint8_t *in, int64_t len) {
+        bytes.init(in, len);
+        left = len;
+        now = -1;
+        next = take();
+        next2 = take();
+    }
+
+    __device__ __forceinline__ uint32_t advance() {
+        now = next;
+        next = next2;
+        next2 = take();
+        return (uint32_t)now;
+    }
+};
+
+// Simulate one input with a whole warp, by stepper w (WarpNfa, or SymNfa of
+// sym_device.cuh). All lanes call it with identical arguments and all receive the verdict.
+template <typename Stepper>
+__device__ Verdict simulate_with(Stepper &w, const uint8_t *in, int64_t len) {
     Verdict v{0, 0, 0};
     int ev = w.init_start();
     if (ev == kAccept) {
@@ -581,14 +613,14 @@ __device__ Verdict simulate_warp(const gbfsm_nfa_dev &A, const Rows &R, const ui
         w.cleanup();
         return v;
     }
-    ByteStream bytes;
+    BytesAhead bytes;
     bytes.init(in, len);
     int64_t pos = 0;
     v.examined = len;
     while (pos < len) {
-        const uint32_t sym = bytes.next();
         ++pos;
-        ev = w.step(sym);
+        const uint32_t sym = bytes.advance();
+        ev = w.step(sym, bytes.next, bytes.next2);
         if (ev == kDead) {
             v.examined = pos;
             break;
@@ -602,6 +634,15 @@ __device__ Verdict simulate_warp(const gbfsm_nfa_dev &A, const Rows &R, const ui
     }
     w.cleanup();
     return v;
+}
+
+// The same with the member-by-member stepper. `R` may point at shared-memory copies of the
+// edge rows.
+template <bool kStaged>
+__device__ Verdict simulate_warp(const gbfsm_nfa_dev &A, const Rows &R, const uint8_t *in,
+                                 int64_t len, WarpScratch S) {
+    WarpNfa<kStaged> w(A, R, S);
+    return simulate_with(w, in, len);
 }
 
 }  // namespace gbfsm

@@ -27,6 +27,7 @@
 #include "dfa_device.cuh"
 #include "engine.hpp"
 #include "nfa_device.cuh"
+#include "sym_device.cuh"
 
 namespace gbfsm {
 namespace {
@@ -58,6 +59,20 @@ PersistLayout persist_layout(int32_t max_words, const gbfsm_plan &p) {
     L.smem_per_warp = L.wbytes + 32u * (uint32_t)max(L.C, 32);
     L.global_per_warp = 3u * (size_t)L.wbytes;
     return L;
+}
+
+// The symbol-list steppers, out of line: they need few registers, and inlined beside the
+// member-by-member ones they made those spill.
+__device__ __noinline__ void sym_chunk(const gbfsm_nfa_dev &nfa, const Rows &R,
+                                       const WarpScratch &S, const uint8_t *base, Bounds bd,
+                                       int index, ChunkRecord *rec) {
+    run_chunk<SymNfa>(nfa, R, S, base, bd.b, bd.e, bd.ov_end, index, rec);
+}
+
+__device__ __noinline__ Verdict sym_whole(const gbfsm_nfa_dev &nfa, const Rows &R,
+                                          const WarpScratch &S, const uint8_t *in, int64_t len) {
+    SymNfa w(nfa, R, S);
+    return simulate_with(w, in, len);
 }
 
 __global__ void __launch_bounds__(kMaxBlockThreads, kPersistMinBlocks) persistent_kernel(
@@ -132,6 +147,7 @@ __global__ void __launch_bounds__(kMaxBlockThreads, kPersistMinBlocks) persisten
             R.eps_edges = nfa.eps_edges;
             S.C = (A->technique == GBFSM_TECH_WARP) ? 0 : min(A->list_capacity, L.C);
             if (task.kind == GBFSM_TASK_LANES) continue;  // gbfsm_lanes_run's tasks
+            const bool sym = sym_usable(nfa, L.C);
             // chunk tasks naming chunks outside the table are skipped
             if ((task.kind == GBFSM_TASK_CHUNK || task.kind == GBFSM_TASK_FIXUP) &&
                 (task.first < 0 || task.count < 1 || task.first + task.count > io.n_chunks))
@@ -143,11 +159,15 @@ __global__ void __launch_bounds__(kMaxBlockThreads, kPersistMinBlocks) persisten
                 const int64_t off = offsets[ch.input];
                 if (S.C == 0) S.C = min(L.C, 32);  // speculation keeps small sets listed
                 const Bounds bd = chunk_bounds(io, nfa, data + off, task.first, off);
-                run_chunk(nfa, R, S, data + off, bd.b, bd.e, bd.ov_end, ch.index,
-                          records + task.first);
+                if (sym)
+                    sym_chunk(nfa, R, S, data + off, bd, ch.index, records + task.first);
+                else
+                    run_chunk<WarpNfa<false>>(nfa, R, S, data + off, bd.b, bd.e, bd.ov_end,
+                                              ch.index, records + task.first);
                 continue;
             }
             if (task.kind == GBFSM_TASK_FIXUP) {
+                if (sym && io.sym_fixups) continue;  // gbfsm_sym_fixup_run's tasks
                 const int32_t id = chunks[task.first].input;
                 const int64_t off = offsets[id];
                 const int64_t e = ends ? ends[id] : offsets[id + 1];
@@ -164,7 +184,12 @@ __global__ void __launch_bounds__(kMaxBlockThreads, kPersistMinBlocks) persisten
             const int32_t id = input_ids[task.first];
             const int64_t b = offsets[id];
             const int64_t e = ends ? ends[id] : offsets[id + 1];
-            const Verdict v = simulate_warp<false>(nfa, R, data + b, e - b, S);
+            Verdict v;
+            if (sym) {
+                v = sym_whole(nfa, R, S, data + b, e - b);
+            } else {
+                v = simulate_warp<false>(nfa, R, data + b, e - b, S);
+            }
             if (lane == 0) {
                 flags[id] = v.flag;
                 lens[id] = v.len;
@@ -271,7 +296,7 @@ gbfsm_status launch_persistent(const gbfsm_automaton *table, int32_t n_automata,
         return fail(GBFSM_INVALID_ARG, "persistent workspace too small: %zu < %zu bytes",
                     workspace_bytes, need);
     if (n_tasks <= 0) return GBFSM_OK;
-    ChunkIO io{nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr};
+    ChunkIO io{nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr, 0};
     if (chunk_io) {
         io.chunks = chunk_io->chunks;
         io.records = static_cast<ChunkRecord *>(chunk_io->records);
@@ -280,6 +305,7 @@ gbfsm_status launch_persistent(const gbfsm_automaton *table, int32_t n_automata,
         io.task_count = chunk_io->task_count;
         io.n_chunks = chunk_io->n_chunks;
         io.aut_ids = chunk_io->aut_ids;
+        io.sym_fixups = chunk_io->sym_fixups;
     }
     uint32_t *ticket = static_cast<uint32_t *>(workspace);
     uint8_t *gws = static_cast<uint8_t *>(workspace) + 256;

@@ -170,6 +170,68 @@ def lane_state_records(nfa):
     return recs.astype(np.uint32), ext.astype(np.uint32)
 
 
+SYMBOL_LIST_LIMIT = 256 * 1024  # pairs; 1024 to a byte on average
+SYMBOL_STATES = 1 << 15
+# automata that lanes run (two-byte supersets this small, engine.LANE_PAIR_MEAN) need none
+SYMBOL_PAIR_MEAN = 32.0
+
+
+def _closures(nfa) -> dict[int, np.ndarray]:
+    """The epsilon closure of every state that has epsilon edges."""
+    erp = np.asarray(nfa.eps_row_ptr, dtype=np.int64)
+    etg = np.asarray(nfa.eps_targets, dtype=np.int64)
+    out = {}
+    for s in np.flatnonzero(erp[1:] > erp[:-1]).tolist():
+        seen, todo = {s}, [s]
+        while todo:
+            u = todo.pop()
+            for t in etg[erp[u]:erp[u + 1]].tolist():
+                if t not in seen:
+                    seen.add(t)
+                    todo.append(t)
+        out[s] = np.fromiter(sorted(seen), dtype=np.int64, count=len(seen))
+    return out
+
+
+def symbol_lists(nfa, limit: int = SYMBOL_LIST_LIMIT):
+    """``(row uint32[258], pairs uint32[k])``: for every byte, the (from, to) pairs of its
+    edges, targets closed under epsilon edges (csrc/sym_device.cuh); list 256 is the start
+    closure. None for automata of more than 32768 states or ``limit`` pairs."""
+    n = int(nfa.num_states)
+    if n > SYMBOL_STATES:
+        return None
+    srp = np.asarray(nfa.sym_row_ptr, dtype=np.int64)
+    sym = np.asarray(nfa.sym_symbols, dtype=np.int64)
+    to = np.asarray(nfa.sym_targets, dtype=np.int64)
+    src = np.repeat(np.arange(n, dtype=np.int64), np.diff(srp))
+    wild = sym == ANY_SYMBOL
+    if int((~wild).sum()) + 256 * int(wild.sum()) > limit:
+        return None
+    closure = _closures(nfa)
+    if closure:  # edges to a state with epsilon edges lead to its closure
+        size = np.ones(n, dtype=np.int64)
+        for s, c in closure.items():
+            size[s] = c.size
+        count = size[to]
+        if int(count[~wild].sum()) + 256 * int(count[wild].sum()) > limit:
+            return None
+        src, sym = np.repeat(src, count), np.repeat(sym, count)
+        to = np.concatenate([closure.get(t, np.array([t])) for t in to.tolist()] +
+                            [np.zeros(0, np.int64)]).astype(np.int64)
+        wild = sym == ANY_SYMBOL
+    c = np.concatenate([sym[~wild], np.repeat(np.arange(256), int(wild.sum()))])
+    src = np.concatenate([src[~wild], np.tile(src[wild], 256)])
+    to = np.concatenate([to[~wild], np.tile(to[wild], 256)])
+    start = int(nfa.start_state)
+    first = closure.get(start, np.array([start], dtype=np.int64))
+    key = np.unique(np.concatenate([(c << 30) | (src << 15) | to, (256 << 30) | first]))
+    row = np.searchsorted(key, np.arange(258, dtype=np.int64) << 30)
+    acc = np.asarray(nfa.accept, dtype=bool)
+    src, to = (key >> 15) & 0x7FFF, key & 0x7FFF
+    pairs = src | (to << 15) | (acc[to].astype(np.int64) << 30)
+    return row.astype(np.uint32), pairs.astype(np.uint32)
+
+
 def slot_table(nfa):
     """The slot table of an epsilon-free NFA (csrc/slots.cu): a dict of ``slots``, ``pairs``
     (uint32), ``state_code`` (uint32 [n]), ``sets`` (uint32 [k, 3]: code, list, size),
@@ -304,6 +366,17 @@ class DeviceNFA:
                 else:
                     self._upload_lane_records(d, lane, precs[:, 0], ssy, nfa, dev)
             d.pair_row = self.pair_row.data_ptr()
+        lists = symbol_lists(nfa) if self.pair_mean > SYMBOL_PAIR_MEAN else None
+        self.sym_pairs = 0 if lists is None else int(lists[1].size)
+        if lists is not None:
+            with torch.cuda.device(dev):
+                self.sym_list_row = torch.from_numpy(lists[0].view(np.int32)).to(dev)
+                self.sym_lists = _padded(max(1, lists[1].size), 4, dev)
+                if lists[1].size:
+                    self.sym_lists[: lists[1].nbytes].copy_(
+                        torch.from_numpy(lists[1].view(np.uint8)))
+            d.sym_lists = self.sym_lists.data_ptr()
+            d.sym_list_row = self.sym_list_row.data_ptr()
         self.desc = d
 
     def _upload_slots(self, d, table, pair_states, srp, nfa, dev) -> None:

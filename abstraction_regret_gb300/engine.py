@@ -350,6 +350,7 @@ class DevicePlan:
         if task_count_word is not None:
             io.task_count = self._hdr(task_count_word)
         io.lane_stage, io.lane_stage_bytes = self.engine.lane_stage
+        io.sym_fixups = int(self.engine.sym_chunked)
         return io
 
     def launch(self, data_ptr: int, d_off, d_ends, d_flags, d_lens, d_examined, stream,
@@ -433,7 +434,21 @@ class DevicePlan:
 
         persist("persistent", self.tasks_persist, self.cap_persist, native.PLAN_PERSIST_TASKS)
         persist("overflow", self.overflow.data_ptr(), self.cap_chunks, native.PLAN_OVERFLOW)
-        persist("fixup", self.tasks_fixup, self.cap_fixup, native.PLAN_FIXUP_TASKS)
+        if eng.sym_chunked:  # a CTA per input of the automata with symbol lists
+            mark("sym_fixup")
+            cio = self.chunk_io(native.PLAN_FIXUP_TASKS)
+            st = lib.gbfsm_sym_fixup_run(
+                table, n_aut, eng.max_words, self.tasks_fixup, int(self.cap_fixup), data_ptr,
+                d_off.data_ptr(), d_ends.data_ptr() if d_ends is not None else None,
+                ctypes.byref(cio), ctypes.byref(eng.plan), d_flags.data_ptr(), d_lens.data_ptr(),
+                d_examined.data_ptr() if d_examined is not None else None, stream.cuda_stream)
+            native.check(st, "gbfsm_sym_fixup_run")
+            mark("sym_fixup")
+            launches += 1
+        if eng.warp_chunked:
+            persist("fixup", self.tasks_fixup, self.cap_fixup, native.PLAN_FIXUP_TASKS)
+        else:
+            launches -= 1
         if chunked_dfa:
             dfa_chunks("dfa_fixup", self.tasks_dfa_fixup, self.cap_dfa_fixup,
                        native.PLAN_DFA_FIXUPS, native.TASK_DFA_FIXUP)
@@ -531,6 +546,13 @@ class PersistentEngine:
             self.table = torch.from_numpy(raw).to(self.device)
             props = torch.cuda.get_device_properties(self.device)
         self.sm_count = props.multi_processor_count
+        # automata whose warps step by symbol lists (sym_usable in csrc/sym_device.cuh), and
+        # whether others' inputs are chunked too
+        sym = np.array([k is Kind.NFA and d.sym_pairs > 0 and
+                        d.num_words * 8 <= 32 * max(self.plan.list_capacity, 32)
+                        for k, d in zip(self.kinds, self.dev)], dtype=bool)
+        self.sym_chunked = bool((sym & self.can_chunk).any())
+        self.warp_chunked = bool((~sym & self.can_chunk).any()) or not self.sym_chunked
         # a pool of one NFA whose slot table fits: the lane launch stages it
         self.lane_stage = ((self.dev[0].stage, self.dev[0].stage_bytes)
                            if len(self.dev) == 1 and isinstance(self.dev[0], DeviceNFA) else (0, 0))

@@ -73,6 +73,8 @@ class NfaDev(ctypes.Structure):
         ("accept_code", ctypes.c_uint32),
         ("multi_code", ctypes.c_uint32),
         ("start_code", ctypes.c_uint32),
+        ("sym_lists", ctypes.c_void_p),
+        ("sym_list_row", ctypes.c_void_p),
     ]
 
 
@@ -137,7 +139,8 @@ class ChunkIO(ctypes.Structure):
                 ("overflow_tasks", ctypes.c_void_p), ("overflow_count", ctypes.c_void_p),
                 ("task_count", ctypes.c_void_p), ("n_chunks", ctypes.c_int32),
                 ("aut_ids", ctypes.c_void_p), ("lane_stage", ctypes.c_int32),
-                ("lane_stage_bytes", ctypes.c_int32), ("lane_share", ctypes.c_int32)]
+                ("lane_stage_bytes", ctypes.c_int32), ("lane_share", ctypes.c_int32),
+                ("sym_fixups", ctypes.c_int32)]
 
 
 LANE_STAGE_NONE, LANE_STAGE_WIDE, LANE_STAGE_NARROW = range(3)  # GBFSM_LANE_STAGE_*
@@ -230,6 +233,8 @@ SIGNATURES: dict[str, tuple] = {
     "gbfsm_slots_build": (_i32, [_i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _i64, _vp,
                                  _vp]),
     "gbfsm_lanes_stage_limit": (_i32, []),
+    "gbfsm_sym_fixup_run": (ctypes.c_int, [_vp, _i32, _i32, _vp, _i32, _vp, _vp, _vp,
+                                           _P(ChunkIO), _P(Plan), _vp, _vp, _vp, _vp]),
     "gbfsm_workload_walk": (_i32, [_i32, _vp, _vp, _vp, _vp, _i32, _vp, _i32, _u64, _vp, _i32]),
     "gbfsm_lanes_run_range": (ctypes.c_int, [_vp, _i32, _vp, _i32, _vp, _vp, _vp, _P(ChunkIO),
                                              _vp]),

@@ -146,6 +146,13 @@ typedef struct gbfsm_nfa_dev {
     uint32_t accept_code; /* codes from here on accept, up to multi_code */
     uint32_t multi_code;
     uint32_t start_code;
+    /* Optional (NULL = warps step a set member by member): symbol lists, for automata of at
+     * most 32768 states. sym_lists[sym_list_row[c] .. sym_list_row[c + 1]) for byte c: a
+     * pair from | to << 15 | accept(to) << 30 for every edge from -c-> t (or ANY) and every
+     * `to` in the epsilon closure of t, without duplicates; list 256: the closure of the
+     * start state (from is 0). sym_list_row has 258 entries. */
+    const uint32_t *sym_lists;
+    const uint32_t *sym_list_row;
 } gbfsm_nfa_dev;
 
 #define GBFSM_CODE_SET (1u << 11) /* info bit of a set's entry in code_recs */
@@ -353,6 +360,8 @@ typedef struct gbfsm_chunk_io {
                                      slot_narrow, each array padded to 16 bytes) */
     int32_t lane_share;           /* lane launches that run side by side (slices of a batch,
                                      each with its range); 0 or 1: this one alone */
+    int32_t sym_fixups;           /* not 0: gbfsm_persistent_run leaves FIXUP tasks of automata
+                                     with symbol lists to gbfsm_sym_fixup_run */
 } gbfsm_chunk_io;
 
 #define GBFSM_LANE_STAGE_NONE 0
@@ -423,6 +432,17 @@ int32_t gbfsm_slots_build(int32_t num_states, const int32_t *sym_row_ptr,
 
 /* Largest gbfsm_chunk_io.lane_stage_bytes of the lane launch on the current device. */
 int32_t gbfsm_lanes_stage_limit(void);
+
+/* Run the FIXUP tasks of automata with symbol lists (others are skipped), a CTA per input:
+ * min(*chunk_io->task_count, n_tasks) tasks when that is non-NULL, else n_tasks. The other
+ * arguments as gbfsm_persistent_run's (plan: the same, its list capacity decides which
+ * automata use their lists). No counterpart in the reference. */
+gbfsm_status gbfsm_sym_fixup_run(const gbfsm_automaton *table, int32_t n_automata,
+                                 int32_t max_words, const gbfsm_task *tasks, int32_t n_tasks,
+                                 const uint8_t *data, const int64_t *offsets,
+                                 const int64_t *ends, const gbfsm_chunk_io *chunk_io,
+                                 const gbfsm_plan *plan, int32_t *flags, int32_t *lens,
+                                 int32_t *examined, void *stream);
 
 /* Resident warps per SM of the lane launch on the current device (0 when it cannot run):
  * a batch whose LANES tasks fit sm_count times this runs in one wave. No counterpart in
