@@ -40,7 +40,7 @@ namespace gbfsm {
 namespace {
 
 constexpr int kPlanThreads = 1024;
-constexpr int kBuckets = 64;
+constexpr int kBuckets = 64;  // (two per lane of the warp that lays them out)
 constexpr int kLaneGroup = 32;
 constexpr int64_t kMaxChunk = 1 << 20;
 // L2 gather rate x time of a dependent lookup / lookups of a collapse per byte of the
@@ -194,13 +194,13 @@ __device__ __forceinline__ int32_t dfa_group(const gbfsm_batch_plan_args &a, int
 __global__ void __launch_bounds__(kPlanThreads) plan_scan_kernel(gbfsm_batch_plan_args a,
                                                                  PlanScratch s) {
     __shared__ int64_t red[6 * 32 + 1];
-    __shared__ int32_t h_work[kBuckets], h_dfa[kBuckets], h_grp[kBuckets];
+    __shared__ int32_t h_work[kBuckets], h_dfa[kBuckets];
     __shared__ int32_t bad;
     const int32_t n = a.n_inputs;
     const int64_t per = ((int64_t)n + kPlanThreads - 1) / kPlanThreads;
     const int32_t lo = (int32_t)min((int64_t)n, (int64_t)threadIdx.x * per);
     const int32_t hi = (int32_t)min((int64_t)n, (int64_t)lo + per);
-    for (int b = threadIdx.x; b < kBuckets; b += blockDim.x) h_work[b] = h_dfa[b] = h_grp[b] = 0;
+    for (int b = threadIdx.x; b < kBuckets; b += blockDim.x) h_work[b] = h_dfa[b] = 0;
     if (threadIdx.x == 0) bad = 0;
     __syncthreads();
 
@@ -385,22 +385,28 @@ __global__ void __launch_bounds__(kPlanThreads) plan_scan_kernel(gbfsm_batch_pla
     // 4. bucket tables and the header (one warp)
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
+        // two buckets a lane, longest first: b1 = 63 - 2 lane, then b1 - 1
+        const int b1 = kBuckets - 1 - 2 * lane, b0 = b1 - 1;
+        const int32_t dfa1 = h_dfa[b1], dfa0 = h_dfa[b0];
+        const int32_t d_incl = (int32_t)warp_inclusive_scan((uint32_t)(dfa1 + dfa0));
+        const int32_t d = __shfl_sync(GBFSM_FULL_MASK, d_incl, 31);  // DFA inputs
+        const int32_t group = max(dfa_group(a, d), 1);
+        const int32_t d1 = d_incl - dfa1 - dfa0, d0 = d1 + dfa1;  // first DFA positions
+        auto groups_before = [&](int32_t x) { return (x + group - 1) / group; };
+        const int32_t grp1 = groups_before(d0) - groups_before(d1);
+        const int32_t grp0 = groups_before(d_incl) - groups_before(d0);
+        const int32_t w1 = h_work[b1], w0 = h_work[b0];
+        const int32_t t_incl = (int32_t)warp_inclusive_scan((uint32_t)(w1 + grp1 + w0 + grp0));
+        const int32_t t = __shfl_sync(GBFSM_FULL_MASK, t_incl, 31);  // persistent tasks
+        const int32_t t1 = t_incl - w1 - grp1 - w0 - grp0, t0 = t1 + w1 + grp1;
+        s.dbase[b1] = d1;
+        s.dbase[b0] = d0;
+        s.tbase[b1] = t1;
+        s.tdfa[b1] = t1 + w1;
+        s.tbase[b0] = t0;
+        s.tdfa[b0] = t0 + w0;
         if (lane == 0) {
-            int32_t d = 0, t = 0, n_dfa = 0;
-            for (int b = 0; b < kBuckets; ++b) n_dfa += h_dfa[b];
-            const int32_t group = max(dfa_group(a, n_dfa), 1);
-            for (int b = kBuckets - 1; b >= 0; --b) {  // DFA positions, longest bucket first
-                s.dbase[b] = d;
-                const int32_t g0 = (d + group - 1) / group;
-                d += h_dfa[b];
-                h_grp[b] = (d + group - 1) / group - g0;
-            }
             s.dbase[kBuckets] = d;
-            for (int b = kBuckets - 1; b >= 0; --b) {  // persistent slots, longest first
-                s.tbase[b] = t;
-                s.tdfa[b] = t + h_work[b];
-                t += h_work[b] + h_grp[b];
-            }
             const int64_t n_lane_tasks = (n_lane + kLaneGroup - 1) / kLaneGroup;
             const bool over = n_chunks + 1 > a.cap_chunks || n_lane_tasks > a.cap_lane_tasks ||
                               t > a.cap_persist_tasks || n_split > a.cap_fixup_tasks ||

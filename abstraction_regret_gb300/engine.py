@@ -432,7 +432,11 @@ class DevicePlan:
             native.check(st, "gbfsm_persistent_run")
             mark(name)
 
-        persist("persistent", self.tasks_persist, self.cap_persist, native.PLAN_PERSIST_TASKS)
+        if eng.persist_tasks:
+            persist("persistent", self.tasks_persist, self.cap_persist,
+                    native.PLAN_PERSIST_TASKS)
+        else:
+            launches -= 1
         persist("overflow", self.overflow.data_ptr(), self.cap_chunks, native.PLAN_OVERFLOW)
         if eng.sym_chunked:  # a CTA per input of the automata with symbol lists
             mark("sym_fixup")
@@ -574,6 +578,8 @@ class PersistentEngine:
             else:
                 cls.append(native.PLAN_NFA_WHOLE)
         self.aut_class = torch.tensor(cls, dtype=torch.int32, device=self.device)
+        # a pool whose inputs are all lane chunks gives the persistent launch no tasks
+        self.persist_tasks = chunk_bytes is None or any(c != native.PLAN_NFA_LANES for c in cls)
         nfa_ix = [i for i, k in enumerate(self.kinds) if k is Kind.NFA]
         small_starts = bool(nfa_ix) and all(
             bool(self.lane_ok[i]) and self.dev[i].pair_mean <= 1.0 for i in nfa_ix)
