@@ -419,4 +419,36 @@ __device__ __forceinline__ bool slot_chunk(const gbfsm_nfa_dev &A, const Table &
     return fits;
 }
 
+// One lane: a whole input from the start state. False (no verdict) when a set outgrows the
+// lane.
+template <typename Table>
+__device__ __forceinline__ bool slot_whole(const gbfsm_nfa_dev &A, const Table &T,
+                                           const uint8_t *in, int64_t len, Verdict &v) {
+    const SlotCodes K{A.set_code, A.accept_code, A.multi_code,
+                      reinterpret_cast<const uint4 *>(A.code_recs)};
+    uint32_t set[kSlotMembers];
+    SlotRun run{A.start_code, 1, set};
+    v = Verdict{0, 0, len};
+    if (A.start_code >= K.accept_begin) {
+        v = Verdict{1, 0, 0};
+        return true;
+    }
+    if (len <= 0) return true;
+    WordStream words;
+    words.init(in, in + len);
+    for (int64_t pos = 0; pos < len; pos += 4) {
+        uint32_t w = words.next_word();
+        if (len - pos >= 4 && slot_word(T, K, run, w)) continue;
+        for (int t = 0; t < 4 && pos + t < len; ++t, w >>= 8) {
+            const int ev = slot_step(T, K, run, w & 0xffu);
+            if (ev == kSlotAlive) continue;
+            if (ev == kSlotFull) return false;
+            const int64_t at = pos + t + 1;
+            v = ev == kSlotAccept ? Verdict{1, (int32_t)at, at} : Verdict{0, 0, at};
+            return true;
+        }
+    }
+    return true;
+}
+
 }  // namespace gbfsm
