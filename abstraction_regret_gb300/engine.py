@@ -32,6 +32,7 @@ from __future__ import annotations
 import ctypes
 import math
 import time
+from contextlib import nullcontext
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -459,9 +460,10 @@ class DevicePlan:
             launches += 1
         return launches + 3
 
-    def fetch_header(self, stream) -> None:
-        """Enqueue the header's copy to pinned host memory (read it after the stream)."""
-        with torch.cuda.stream(stream):
+    def fetch_header(self, stream, current: bool = False) -> None:
+        """Enqueue the header's copy to pinned host memory (read it after the stream).
+        ``current``: ``stream`` is the current one."""
+        with nullcontext() if current else torch.cuda.stream(stream):
             self.h_header.copy_(self.header, non_blocking=True)
 
     def check(self) -> None:
@@ -954,7 +956,7 @@ class PersistentEngine:
         d_aut = self.upload_aut_ids(aut_ids, stream)
         d_data, d_off, h_off, total = self._staging.put(inputs, stream,
                                                         defer=self.pipeline_parts > 1,
-                                                        lengths=lengths)
+                                                        lengths=lengths, current=True)
         self._results.ensure(max(n, 1))
         res = self._results
         e0 = torch.cuda.Event(enable_timing=True)
@@ -976,9 +978,9 @@ class PersistentEngine:
             plan.launch(d_data.data_ptr(), d_off, None, res.d[0], res.d[1],
                         res.d[2] if with_examined else None, stream)
         e1.record(stream)
-        res.fetch(n, stream)
+        res.fetch(n, stream, 3 if with_examined else 2, current=True)
         if n:
-            plan.fetch_header(stream)
+            plan.fetch_header(stream, current=True)
         if idle is not None:
             idle()
         stream.synchronize()

@@ -105,15 +105,16 @@ class _BatchExecutor:
         e1 = torch.cuda.Event(enable_timing=True)
         if self.end_to_end:
             e0.record(stream)
-        d_data, d_off, _, _ = self._staging.put(inputs, stream, lengths=lengths)
+        d_data, d_off, _, _ = self._staging.put(inputs, stream, lengths=lengths, current=True)
         self._results.ensure(max(n, 1))
         r = self._results
         if not self.end_to_end:
             e0.record(stream)
-        self._launch(d_data, d_off, n, r.d[0], r.d[1], r.d[2] if with_examined else None, stream)
+        d = r.d
+        self._launch(d_data, d_off, n, d[0], d[1], d[2] if with_examined else None, stream)
         if not self.end_to_end:
             e1.record(stream)
-        r.fetch(n, stream)
+        r.fetch(n, stream, 3 if with_examined else 2, current=True)
         if self.end_to_end:
             e1.record(stream)
         if idle is not None:
