@@ -78,16 +78,21 @@ constexpr int kPollEveryStep = 512;   // set size above which every bitmap step 
 constexpr int kMeetBytes = 4;  // bytes between two removals of members that have met
 constexpr int kListMembers = 1024;    // members from which a set is kept as a list
 
+// (the latch lies in global memory, or in shared memory for a CTA's own input)
+__device__ __forceinline__ int32_t read_latch(const int32_t *latch) {
+    return *static_cast<const volatile int32_t *>(latch);
+}
+
 // True when a chunk of index below `index` has latched the input (latch may be NULL).
 __device__ __forceinline__ bool latched_below(const int32_t *latch, int32_t index) {
-    return latch && __ldcv(latch) < index;
+    return latch && read_latch(latch) < index;
 }
 
 // The same for the whole warp (latch and index warp-uniform): lane 0 reads the latch and
 // every lane gets its answer, so the warp leaves a collective walk together.
 __device__ __forceinline__ bool warp_latched_below(const int32_t *latch, int32_t index) {
     if (!latch) return false;
-    int32_t v = lane_id() == 0 ? __ldcv(latch) : 0;
+    int32_t v = lane_id() == 0 ? read_latch(latch) : 0;
     v = __shfl_sync(GBFSM_FULL_MASK, v, 0);
     return v < index;
 }

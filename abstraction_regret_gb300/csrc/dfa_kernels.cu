@@ -242,6 +242,12 @@ gbfsm_status launch_dfa_walk(const gbfsm_dfa_dev &d, const gbfsm_plan &p, const 
                     threads);
     const size_t budget = (size_t)smem_optin() - kSmemReserve;
     const bool staged = p.stage && (16u + (size_t)pad16(d.table_bytes) <= budget);
+    // a table too large for one CTA and no more inputs than warps: the inputs cut into chunks
+    // (4096 inputs of 64 KiB on 4096 states: 12.6 ms by the cluster's one chain per input)
+    gbfsm_status split;
+    if (p.stage && !staged && p.block_threads <= 0 &&
+        launch_dfa_split(d, data, offsets, n_inputs, flags, lens, examined, stream, split))
+        return split;
     // a 2-byte table too large for one CTA: split over the CTAs of a cluster
     const int ctas = (int)((d.num_states + (1 << kSliceStatesLog2) - 1) >> kSliceStatesLog2);
     if (p.stage && !staged && d.entry_bytes == 2 && ctas >= 2 && ctas <= kMaxClusterCtas &&

@@ -65,6 +65,10 @@ gbfsm_status launch_nfa_bitmap(const gbfsm_nfa_dev &a, const BitmapPlan &bp, con
 gbfsm_status launch_dfa_walk(const gbfsm_dfa_dev &d, const gbfsm_plan &p, const uint8_t *data,
                              const int64_t *offsets, int32_t n_inputs, int32_t *flags,
                              int32_t *lens, int32_t *examined, cudaStream_t stream);
+// False (nothing launched) when the inputs do not fit one wave of it.
+bool launch_dfa_split(const gbfsm_dfa_dev &d, const uint8_t *data, const int64_t *offsets,
+                      int32_t n_inputs, int32_t *flags, int32_t *lens, int32_t *examined,
+                      cudaStream_t stream, gbfsm_status &status);
 gbfsm_status launch_persistent(const gbfsm_automaton *table, int32_t n_automata,
                                int32_t max_words,
                                const gbfsm_task *tasks, int32_t n_tasks, const int32_t *input_ids,

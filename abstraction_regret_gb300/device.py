@@ -483,11 +483,13 @@ class DeviceDFA:
             code = int(err[0].item())
             if code:
                 raise ValueError(f"invalid DFA: a successor is outside [0, {n}) (code {code})")
+            # table entries that lead to an accepting state (successors are checked by now)
+            accepting = int((a_dev[:n] != 0)[t_dev[: n * ALPHABET].long()].sum().item())
         d = native.DfaDev()
         d.num_states = n
         d.start_state = start
         d.entry_bytes = entry_bytes
-        d.flags = 0
+        d.flags = native.DFA_RARE_ACCEPT if accepting * 50000 <= n * ALPHABET else 0
         d.table = self.table.data_ptr()
         d.accept_bits = self.accept_bits.data_ptr()
         d.table_bytes = self.table_bytes

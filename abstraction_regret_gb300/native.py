@@ -32,6 +32,7 @@ EDGE_SYMBOL_MASK = 0x1FF
 EDGE_ACCEPT = 1 << 9
 EDGE_HAS_EPS = 1 << 10
 CODE_SET = 1 << 11  # GBFSM_CODE_SET
+DFA_RARE_ACCEPT = 1  # GBFSM_DFA_RARE_ACCEPT
 
 FLAG_TIMEOUT = -1
 

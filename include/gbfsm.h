@@ -164,11 +164,15 @@ typedef struct gbfsm_dfa_dev {
     int32_t num_states;
     int32_t start_state;
     int32_t entry_bytes; /* 2 or 4 */
-    int32_t flags;
+    int32_t flags;       /* GBFSM_DFA_* */
     const void *table;
     const uint32_t *accept_bits;
     uint64_t table_bytes;
 } gbfsm_dfa_dev;
+
+/* At most one table entry in 50000 leads to an accepting state: a run over uniform bytes
+ * goes on for tens of thousands (a hint for how to launch; results do not depend on it). */
+#define GBFSM_DFA_RARE_ACCEPT 1
 
 /* How to run a batch. Zero fields select the defaults. */
 typedef struct gbfsm_plan {

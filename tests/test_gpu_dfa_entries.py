@@ -70,3 +70,55 @@ def test_few_and_many_short_inputs():
     for n in (3, 6000):
         _check(dfa, [rng.integers(0, 256, int(k), dtype=np.uint8).tobytes()
                      for k in rng.integers(0, 400, n)])
+
+
+def _plain(dfa, inputs):
+    """One plain launch (the default technique) against the oracle, examined bytes too."""
+    from abstraction_regret_gb300.executors import CudaDFAExecutor
+
+    f, l, e, _, _ = CudaDFAExecutor(dfa).run_arrays(inputs, with_examined=True)
+    data, off = O.flatten(inputs)
+    of, ol, oe = O.dfa_batch(dfa, data, off)
+    assert np.array_equal(f, of) and np.array_equal(l, ol) and np.array_equal(e, oe)
+    return of
+
+
+@pytest.mark.parametrize("states,n_inputs", [(500, 3), (500, 700), (1000, 1500), (1000, 4500),
+                                             (600, 2500), (5000, 40)])
+def test_plain_launch_cuts_inputs(states, n_inputs):
+    """4, 2 or 1 warps per input by their number, and more inputs than one wave (no cut);
+    lengths around one, two and eight chunks; an alarm byte at the cuts and elsewhere."""
+    rng = np.random.default_rng(states + n_inputs)
+    trans = rng.integers(0, states - 2, size=(states, 256), dtype=np.int32)
+    trans[7, 255] = states - 2   # two steps to the accepting state: few entries lead there
+    trans[:, 254] = 7
+    trans[states - 2, 253] = states - 1
+    accept = np.arange(states) == states - 1
+    dfa = DFA(num_states=states, start_state=0, accept=accept, trans=trans.reshape(-1))
+    chunk = max(256, 2 * states)
+    lengths = np.r_[0, 1, 15, 16, chunk, 2 * chunk - 1, 2 * chunk, 2 * chunk + 1, 8 * chunk,
+                    9 * chunk + 5, rng.integers(0, 5 * chunk, 60)]
+    inputs = []
+    for i in range(n_inputs):
+        n = int(lengths[i % lengths.size]) if n_inputs < 3000 else int(rng.integers(0, 600))
+        x = rng.integers(0, 250, n, dtype=np.uint8)
+        if n > 8 and i % 2:
+            prefix = min(1024, n // 16)
+            at = [prefix, prefix + (n - prefix) // 2, int(rng.integers(0, n - 3)), n - 3]
+            k = min(max(at[i // 2 % 4] - int(rng.integers(0, 4)), 0), n - 3)
+            x[k:k + 3] = (254, 255, 253)
+        inputs.append(x.tobytes())
+    flags = _plain(dfa, inputs)
+    if n_inputs > 10:  # (the first three are too short for the alarm)
+        assert 0 < int(flags.sum()) < len(inputs)
+
+
+@pytest.mark.parametrize("states", [500, 3000])
+def test_plain_launch_of_a_dfa_that_accepts_at_once(states):
+    """The start state accepts: an empty walk, whatever the length."""
+    dfa = random_dfa(states, accept_prob=0.0, seed=states)
+    acc = dfa.accept.copy()
+    acc[0] = True
+    dfa = DFA(num_states=states, start_state=0, accept=acc,
+              trans=np.where(dfa.trans == 0, 1, dfa.trans).astype(np.int32))
+    _plain(dfa, [bytes(n) for n in (0, 1, 100, 30000)])
