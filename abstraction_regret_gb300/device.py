@@ -215,10 +215,13 @@ def symbol_lists(nfa, limit: int = SYMBOL_LIST_LIMIT):
         count = size[to]
         if int(count[~wild].sum()) + 256 * int(count[wild].sum()) > limit:
             return None
-        src, sym = np.repeat(src, count), np.repeat(sym, count)
-        to = np.concatenate([closure.get(t, np.array([t])) for t in to.tolist()] +
-                            [np.zeros(0, np.int64)]).astype(np.int64)
-        wild = sym == ANY_SYMBOL
+        more = np.flatnonzero(count > 1)
+        if more.size:  # (these edges alone: an automaton has few of them)
+            one = count == 1
+            src = np.concatenate([src[one], np.repeat(src[more], count[more])])
+            sym = np.concatenate([sym[one], np.repeat(sym[more], count[more])])
+            to = np.concatenate([to[one]] + [closure[t] for t in to[more].tolist()])
+            wild = sym == ANY_SYMBOL
     c = np.concatenate([sym[~wild], np.repeat(np.arange(256), int(wild.sum()))])
     src = np.concatenate([src[~wild], np.tile(src[wild], 256)])
     to = np.concatenate([to[~wild], np.tile(to[wild], 256)])
