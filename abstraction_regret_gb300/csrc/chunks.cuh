@@ -732,7 +732,8 @@ struct LinkView {
     int2 end;      // dead_at, end_count
     int64_t begin;
 };
-static_assert(kCheckpoints == 6 && sizeof(ChunkRecord) % 16 == 0 && offsetof(ChunkRecord, dead_at) == 48 &&
+static_assert(kCheckpoints == 6 && sizeof(ChunkRecord) % 16 == 0 &&
+                  offsetof(ChunkRecord, dead_at) == 48 &&
                   offsetof(ChunkRecord, ov_counts) == 64 && offsetof(ChunkRecord, begin) == 88,
               "the link test loads a record by 16-byte groups");
 

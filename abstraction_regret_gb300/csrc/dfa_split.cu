@@ -3,7 +3,7 @@
 // (dfa_chunks.cuh: collapse, walk and fix-up, here with the records in shared memory and a
 // barrier between the three). One thread per input leaves 4096 inputs as 4096 chains of
 // dependent lookups, 0.19-0.23 us each, and the GPU idle; two chunks a warp halve the
-// chain, and fewer inputs get more. 4096 inputs of 64 KiB on 4096 states: 7.8 ms against
+// chain, and fewer inputs get more. 4096 inputs of 64 KiB on 4096 states: 7.4 ms against
 // 12.6 ms by dfa_cluster_kernel; 136 inputs of up to 4 KiB on 524 states 0.23 against 0.63.
 #include <map>
 #include <mutex>

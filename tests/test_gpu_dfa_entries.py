@@ -122,3 +122,23 @@ def test_plain_launch_of_a_dfa_that_accepts_at_once(states):
     dfa = DFA(num_states=states, start_state=0, accept=acc,
               trans=np.where(dfa.trans == 0, 1, dfa.trans).astype(np.int32))
     _plain(dfa, [bytes(n) for n in (0, 1, 100, 30000)])
+
+
+@pytest.mark.parametrize("states", [64, 3000])
+def test_every_alignment_and_tail(states):
+    """Inputs of 0 to 70 bytes packed behind one another, so that a warp's lanes start at
+    every offset of a 16-byte block and end at every other; one accept at a random byte."""
+    rng = np.random.default_rng(states)
+    trans = rng.integers(0, states - 1, size=(states, 256), dtype=np.int32)
+    trans[:, 255] = states - 1
+    dfa = DFA(num_states=states, start_state=0, accept=np.arange(states) == states - 1,
+              trans=trans.reshape(-1))
+    inputs = []
+    for k in range(71 * 17):
+        x = rng.integers(0, 255, k % 71, dtype=np.uint8)
+        if x.size and k % 3 == 0:
+            x[int(rng.integers(0, x.size))] = 255
+        inputs.append(x.tobytes())
+    flags = _plain(dfa, inputs)
+    assert 0 < int(flags.sum()) < len(inputs)
+    _check(dfa, inputs)
