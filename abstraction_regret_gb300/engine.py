@@ -78,9 +78,9 @@ DFA_OVERLAP_CHUNKS = 1.0
 # a host batch the device gathers in place (staging.py) of at least PIPELINE_MIN_BYTES is
 # gathered in PIPELINE_PARTS slices of contiguous inputs, each slice's lane tasks starting
 # as soon as its bytes are in (run_requests); PIPELINE_LANE_WAVES as in GraphRunner.
-# Measured per run_batch call on c3-sustained inputs, whole gather / 8 slices: 8 MB 0.75 /
-# 0.90 ms, 32 MB 1.12 / 1.17, 129 MB 2.48 / 2.57, 261 MB 4.47 / 4.23 (the shorter chunks
-# of two lane waves and the extra launches outweigh the overlap below about 160 MiB)
+# Measured per run_batch call on c3-sustained inputs, whole gather / 8 slices: 10 MB 0.52 /
+# 0.66 ms, 31 MB 0.73 / 0.83, 121 MB 1.48 / 1.57, 248 MB 2.59 / 2.64 (the shorter chunks of
+# two lane waves and the extra launches outweigh the overlap; level from about 160 MiB)
 PIPELINE_PARTS = 8
 PIPELINE_MIN_BYTES = 160 << 20
 PIPELINE_LANE_WAVES = 2
@@ -1045,9 +1045,8 @@ class GraphRunner:
           1 - shrink * k / P: a slice that arrives later has less time left, so its lanes
           get shorter chunks. ``lane_waves`` > 1 cuts the lane chunks shorter, to fill
           that many waves of the lane launch, so that each arriving slice finds free lanes.
-          Measured on c3-sustained (2.76 ms per step): 8 slices, no shrink, 2 waves; one
-          wave with shrink 0.75 took 2.81 ms, 4 waves 2.87 ms (per-chunk work grows: the
-          resident step takes 1.92 / 2.22 / 2.61 ms at 1 / 2 / 4 waves).
+          Measured on c3-sustained: 8 slices, no shrink, 2 waves 1.58 ms per step; 1 wave
+          1.82 ms, 6 slices 1.67, 12 or 16 slices 1.64.
 
         ``kernel_only`` plans and runs the batch on the device copy of the inputs."""
         if ingest not in self.INGEST:

@@ -12,7 +12,7 @@ inputs stay larger than L2 where the case's kernel streams them:
 * ``c2-sustained``   the DFA cluster walk on c2-sustained (4096 x 64 KiB);
 * ``c4-sustained``   the engine on c4-sustained (64 NFAs, 1024 inputs; lanes and
                      persistent launches);
-* ``dfa-long``       chunked DFA walks (``dfa_chunks_kernel``): 8 inputs of 2 MiB on
+* ``dfa-long``       chunked DFA walks (``dfa_collapse_kernel``, ``dfa_walk_chunks_kernel``): 8 inputs of 2 MiB on
                      the c2 DFA (4096 states, no accepting state);
 * ``c5-live``        the serving loop over the c5 pool (16 NFAs, 16 DFAs): the first
                      2000 requests of the live trace, all arriving at once (the oracle

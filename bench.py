@@ -25,8 +25,9 @@ Printed (rank 0, one JSON line):
   dfa         the plain DFA walk on the c2 configuration (4096 states, 4096 x 64 KiB);
   serving     the continuous-batching loop on the c5 trace (p50 / p99 latency, offered
               GB/s, against one plain launch per request);
-  roofline    the dominant kernel (the lane launch) against the measured HBM copy
-              bandwidth, with the input stream alone beside it;
+  roofline    the dominant kernel (the lane launch) against the measured shared-memory
+              rate (its table is staged there; the L2 read bandwidth where it is not), with
+              the input stream against HBM beside it;
   cpu_baseline the CPU oracle port on this host's cores on a bounded sample.
 
 With ``--impl reference`` the reference's CPU algorithm (the C port of
@@ -533,7 +534,9 @@ def main(argv=None) -> int:
                              .get("hbm_gbs", 6800.0)) \
                 if (REPO / "MEASURED_PEAKS.json").exists() else 6800.0
             # per examined symbol: 1 input byte (HBM stream) + one 2-byte table entry read
-            # from on-chip memory; each input is one chain of dependent lookups
+            # from on-chip memory; an input is one chain of dependent lookups, or two where
+            # the launch cuts it (a DFA that rarely accepts)
+            chains2 = int(b2.n_inputs) * (2 if ex2.dev.desc.flags else 1)
             longest = int(np.diff(b2.offsets).max())
             extras[f"dfa_c2_{variant}"] = {
                 "offered_GBps": b2.total_bytes / (d_ms * 1e-3) / 1e9,
@@ -541,11 +544,11 @@ def main(argv=None) -> int:
                 "ms": d_ms, "examined_bytes": int(oe.sum()), "checked": int(of.size),
                 "roofline": {"bound": "latency (one dependent lookup per symbol per input)",
                              "hbm_frac_input_stream": examined_gbps / hbm_peak,
-                             "chains": int(b2.n_inputs),
+                             "chains": chains2,
                              "ns_per_lookup_longest_chain": d_ms * 1e6 / max(1, longest)
                              if variant == "sustained" else None},
                 "cpu_baseline": cpu2,
-                "_counts": {"examined": int(oe.sum()), "chains": int(b2.n_inputs)}}
+                "_counts": {"examined": int(oe.sum()), "chains": chains2}}
             del r2, ex2, b2
     if "run_batch" in sections and rank == 0:
         extras["run_batch_default"] = run_batch_section(batch, flags, lens, steps=3)
@@ -579,9 +582,10 @@ def main(argv=None) -> int:
     hbm = float(peaks.get("hbm_gbs", 6800.0))
     top = max(phase_ms, key=phase_ms.get) if phase_ms else "lanes"
     kernel_ms = phase_ms.get(top, ms)
-    kernel_name = {"lanes": "lanes_kernel", "persistent": "persistent_kernel",
-                   "overflow": "persistent_kernel", "fixup": "persistent_kernel",
-                   "plan": "plan_scan_kernel"}[top]
+    staged = eng.lane_stage[0]
+    kernel_name = {"lanes": "lanes_shared_kernel" if staged else "lanes_kernel",
+                   "persistent": "persistent_kernel", "overflow": "persistent_kernel",
+                   "fixup": "persistent_kernel", "plan": "plan_scan_kernel"}.get(top, top)
     # algorithmic bytes of the exact simulation (CSR view): per examined symbol 1 input
     # byte, per active state an 8-byte row range, per scanned edge 8 bytes (symbol +
     # target); 12 bytes of verdicts per input. Counted by the oracle on the same batch.
@@ -635,6 +639,28 @@ def main(argv=None) -> int:
                 "note": "algorithmic bytes (per symbol: 1 input byte, 8 per active state, 8 "
                         "per scanned edge) are mostly edge gathers from a 1 MiB table held "
                         "in L1/L2; DRAM carries the input stream"}
+
+    if staged and top == "lanes":
+        # the slot table lies in shared memory: an examined symbol of an active state is one
+        # lookup, one 4-byte bank word a load and lane (two loads in the 3-byte form). Held
+        # against the conflict-free shared-memory rate; 32 lanes reading unrelated words
+        # take about 3.5 passes a load (the largest of 32 bins of 32 balls), which is the
+        # rate a random lookup can reach.
+        loads = 2 if staged == 2 else 1
+        words = 4 * loads * gate.get("states_stepped", 0)
+        peak = onchip.get("smem_GBps") if onchip else None
+        rate = words / (kernel_ms * 1e-3) / 1e9
+        roofline.update({
+            "bound": "smem", "achieved": rate, "peak": peak,
+            "frac": rate / peak if peak else None,
+            "peak_source": "measured in this run: conflict-free shared loads (gbfsm_probe_smem)",
+            "loads_per_lookup": loads, "expected_passes_per_load": 3.5,
+            "frac_of_random_lookups": 3.5 * rate / peak if peak else None,
+            "note": "one lookup per examined symbol and active state in a slot table in shared "
+                    "memory, bound by bank conflicts; algorithmic_bytes_per_launch is the CSR "
+                    "view of the same work"})
+        for key in ("gathers", "latency"):
+            roofline.pop(key, None)
 
     if rank == 0:
         line = {"metric": METRIC, "value": value, "unit": "GB/s", "n_gpus": world,
