@@ -486,7 +486,7 @@ gbfsm_status run_nfa_host(int32_t technique, int32_t stage, bool end_to_end,
     if (num_strings > 0 && (!out_flags || !out_lens))
         return fail(GBFSM_INVALID_ARG, "output arrays are NULL");
     DeviceBuffers buf;
-    gbfsm_nfa_dev desc;
+    gbfsm_nfa_dev desc{};  // optional parts absent
     GBFSM_TRY(build_nfa(buf, srp, stg, ssy, erp, etg, accept_bytes, num_states, start_state, &desc));
     Events ev;
     GBFSM_TRY(ev.create());
