@@ -486,13 +486,20 @@ class DeviceDFA:
             code = int(err[0].item())
             if code:
                 raise ValueError(f"invalid DFA: a successor is outside [0, {n}) (code {code})")
-            # table entries that lead to an accepting state (successors are checked by now)
-            accepting = int((a_dev[:n] != 0)[t_dev[: n * ALPHABET].long()].sum().item())
+            # the share of entries that lead to an accepting state (their top bits), for the
+            # paths over 2-byte tables; counted a slice at a time, as a sum over booleans
+            # takes 9 bytes an entry
+            self.accept_share = None
+            if entry_bytes == 2:
+                top = self.table[: 2 * n * ALPHABET].view(torch.int16)
+                accepting = sum((part < 0).sum() for part in top.split(1 << 20))
+                self.accept_share = int(accepting.item()) / (n * ALPHABET)
         d = native.DfaDev()
         d.num_states = n
         d.start_state = start
         d.entry_bytes = entry_bytes
-        d.flags = native.DFA_RARE_ACCEPT if accepting * 50000 <= n * ALPHABET else 0
+        rare = self.accept_share is not None and self.accept_share * 50000 <= 1.0
+        d.flags = native.DFA_RARE_ACCEPT if rare else 0
         d.table = self.table.data_ptr()
         d.accept_bits = self.accept_bits.data_ptr()
         d.table_bytes = self.table_bytes
