@@ -18,6 +18,8 @@ namespace {
 
 constexpr int kDfaChunkThreads = 128;  // 4 warps per CTA
 constexpr int kDfaChunkWarps = kDfaChunkThreads / 32;
+// A third of the time of the chunk's walk while the device has idle warps.
+constexpr uint32_t kBudgetPerByte = 20;
 
 // A task of the list that names a DFA and chunks inside the tables; false otherwise.
 __device__ __forceinline__ bool dfa_task_ok(const gbfsm_task &task,
@@ -58,10 +60,10 @@ __global__ void __launch_bounds__(kDfaChunkThreads, 6) dfa_collapse_kernel(
         int32_t *lt = latch ? latch + ch.input : nullptr;
         if (d.entry_bytes == 2)
             dfa_chunk_collapse<uint16_t>(d, data + off, ch.begin - off, ch.end - off, ch.index,
-                                         bm0, bm1, list, rec, lt);
+                                         bm0, bm1, list, rec, lt, kBudgetPerByte);
         else
             dfa_chunk_collapse<uint32_t>(d, data + off, ch.begin - off, ch.end - off, ch.index,
-                                         bm0, bm1, list, rec, lt);
+                                         bm0, bm1, list, rec, lt, kBudgetPerByte);
         __syncwarp();
     }
 }

@@ -17,9 +17,11 @@
 //    of the entry states of its chunk, whose record gives the state at the next chunk's p,
 //    and so on. The first accept on that path is the input's verdict.
 //
-// A chunk whose set never shrinks to kEntries members has no entry states: the chunk before
-// walks on through it (up to the automaton's dfa_overlap bytes past its own end). Where a
-// walk ends before the next entry position, the fix-up walks the gap.
+// A chunk whose set does not shrink to kEntries members within its bytes and its budget of
+// lookups has no entry states: the chunk before walks on through it (up to the automaton's
+// dfa_overlap bytes past its own end). Where a walk ends before the next entry position, the
+// fix-up walks the gap. The budget (collapse_budget) is what keeps a DFA whose states are
+// permuted by every byte from spending n lookups a byte to its chunks' ends.
 //
 // Early stop: an accept of the first chunk, or one found by every lane of a chunk, is in
 // the input's true walk whatever came before, so the input's verdict lies at or before it.
@@ -111,9 +113,22 @@ __device__ __forceinline__ int32_t warp_sum_i32(int32_t v) {
     return v;
 }
 
+// Lookups that the collapse of a chunk of `len` bytes may take, `per_byte` of them for each
+// byte: twice what a trial of the automaton took (where nothing is known, as if that had been
+// twice a random DFA's), and a share of what the chunk's own walk costs, for texts on which the set
+// shrinks later than on the trial's. One warp makes about 57 set lookups in the time of one
+// step of a walk, and the whole device 30 lookups for every byte that 5000 warps walk.
+__device__ __forceinline__ int32_t collapse_budget(const gbfsm_dfa_dev &d, int64_t len,
+                                                    uint32_t per_byte) {
+    const int64_t known = d.collapse_lookups ? (int64_t)d.collapse_lookups
+                                             : 2 * collapse_schedule((uint32_t)d.num_states);
+    return (int32_t)min(2 * known + (int64_t)per_byte * len, (int64_t)1 << 30);
+}
+
 // The whole warp: walk the set of all n states from position b over bytes [b, e) until it
 // has at most `want` (<= 32) members. Returns that position (lane l < count holds a member
-// in `member`), -1 when the set is still larger at e, or -2 when a chunk below `index` has
+// in `member`), -1 when the set is still larger at e or after `budget` lookups (steps of at
+// most 32 members cost no more than a walk's and are not counted), or -2 when a chunk below `index` has
 // latched the input (latch may be NULL). bm0 / bm1: shared bitmaps of at least ceil(n / 32)
 // words; list: 2 * kListMembers shared 16-bit words. The set is a bitmap while it is large,
 // then a list (a step then costs a lookup, an atomic and a ballot per 32 members, whatever
@@ -123,7 +138,7 @@ template <typename Entry>
 __device__ int64_t dfa_collapse(const Entry *T, uint32_t n, const uint8_t *base, int64_t b,
                                 int64_t e, int want, uint32_t *bm0, uint32_t *bm1,
                                 uint16_t *list, uint32_t &member, int32_t &count,
-                                const int32_t *latch, int32_t index) {
+                                const int32_t *latch, int32_t index, int32_t budget) {
     constexpr uint32_t ACC = EntryTraits<Entry>::kAccept;
     const uint32_t lane = lane_id();
     const uint32_t nw = (n + 31u) >> 5;
@@ -154,6 +169,7 @@ __device__ int64_t dfa_collapse(const Entry *T, uint32_t n, const uint8_t *base,
         }
         __syncwarp();
         pos = b + 1;
+        budget -= (int32_t)n;
         uint32_t *cur = bm1, *nxt = bm0;
         for (uint32_t w = lane; w < nw; w += 32) count += __popc(cur[w]);
         count = warp_sum_i32(count);
@@ -162,6 +178,8 @@ __device__ int64_t dfa_collapse(const Entry *T, uint32_t n, const uint8_t *base,
             if ((count > kPollEveryStep || (pos - b) % kLatchPollSets == 0) &&
                 warp_latched_below(latch, index))
                 return -2;
+            if (budget < 0) return -1;
+            budget -= count;
             const uint32_t c = __ldg(base + pos);
             for (uint32_t w = lane; w < nw; w += 32) nxt[w] = 0u;
             __syncwarp();
@@ -220,8 +238,10 @@ __device__ int64_t dfa_collapse(const Entry *T, uint32_t n, const uint8_t *base,
         bytes.init(base + pos, e - pos);
         while (count > 32 && pos < e) {
             if (++polls % 4 == 0 && warp_latched_below(latch, index)) return -2;
+            if (budget < 0) return -1;
             // up to kMeetBytes bytes, then the members that met are dropped
             const int k = (int)min((int64_t)kMeetBytes, e - pos);
+            budget -= count * k;
             uint32_t c[kMeetBytes];
 #pragma unroll
             for (int j = 0; j < kMeetBytes; ++j) c[j] = j < k ? bytes.next() : 0u;
@@ -296,11 +316,12 @@ __device__ int64_t dfa_collapse(const Entry *T, uint32_t n, const uint8_t *base,
 }
 
 // Collapse of chunk `index` of an input, spanning positions [b, e) of `base` (the input's
-// first byte): its entry position and states, to rec.
+// first byte): its entry position and states, to rec. per_byte: see collapse_budget.
 template <typename Entry>
 __device__ void dfa_chunk_collapse(const gbfsm_dfa_dev &d, const uint8_t *base, int64_t b,
                                    int64_t e, int index, uint32_t *bm0, uint32_t *bm1,
-                                   uint16_t *list, DfaChunkRecord *rec, int32_t *latch) {
+                                   uint16_t *list, DfaChunkRecord *rec, int32_t *latch,
+                                   uint32_t per_byte) {
     const Entry *T = static_cast<const Entry *>(d.table);
     const uint32_t lane = lane_id();
     int64_t p;
@@ -320,7 +341,7 @@ __device__ void dfa_chunk_collapse(const gbfsm_dfa_dev &d, const uint8_t *base, 
         }
     } else {
         p = dfa_collapse<Entry>(T, (uint32_t)d.num_states, base, b, e, kEntries, bm0, bm1, list,
-                                member, count, latch, index);
+                                member, count, latch, index, collapse_budget(d, e - b, per_byte));
     }
     if (lane == 0) {
         rec->p = (int32_t)p;

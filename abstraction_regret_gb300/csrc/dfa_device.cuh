@@ -27,6 +27,13 @@ struct EntryTraits<uint32_t> {
     static constexpr uint32_t kAccept = 0x80000000u;
 };
 
+// Table lookups that walking the set of all n states of a random DFA takes until it has 16
+// members: the set holds about 2n/t states after t bytes, so n + the sum of 2n/t up to n/8.
+__host__ __device__ inline int64_t collapse_schedule(uint32_t n) {
+    const float m = n > 16u ? (float)n : 16.0f;
+    return (int64_t)(2.0f * m * (1.0f + logf(m / 16.0f)));
+}
+
 // Row index type: 32-bit for 2-byte tables (at most 32768 states), 64-bit otherwise.
 template <typename Entry>
 struct RowIndex {

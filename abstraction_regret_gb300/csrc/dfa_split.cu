@@ -18,6 +18,7 @@ namespace {
 
 constexpr int kSplitMaxWarps = 4;
 constexpr int kSplitPerWarp = 32 / kEntries;  // chunks a warp walks
+constexpr uint32_t kBudgetPerByte = 1;  // (this launch fills the device with warps)
 
 // Shortest chunk: a set of n states collapses in about n / 8 bytes, whose steps take a few
 // times a walk's; with chunks of n / 2 bytes, inputs of about n bytes on 8000 states were 9%
@@ -92,7 +93,7 @@ __global__ void __launch_bounds__(kSplitMaxWarps * 32, 7) dfa_split_kernel(
     for (int c = warp == 0 ? warps : warp; c < count; c += warps)
         dfa_chunk_collapse<uint16_t>(d, base, prefix + c * more / count,
                                      prefix + (c + 1) * more / count, c, bm0, bm1, list,
-                                     dfa_record(records, c), latch);
+                                     dfa_record(records, c), latch, kBudgetPerByte);
     __syncthreads();
     const int c = warp + (int)(lane / kEntries) * warps;
     DfaChunkRecord *rec = dfa_record(records, c < count ? c : 0);
@@ -150,10 +151,13 @@ int split_blocks_per_sm(uint32_t words, int warps) {
 bool launch_dfa_split(const gbfsm_dfa_dev &d, const uint8_t *data, const int64_t *offsets,
                       int32_t n_inputs, int32_t *flags, int32_t *lens, int32_t *examined,
                       cudaStream_t stream, gbfsm_status &status) {
-    // a DFA that accepts often ends its inputs within a few thousand bytes, about as many as
+    // A DFA whose set of all states has been seen to shrink as fast as a random one's does:
+    // the cut pays while a collapse takes no more than about twice as many lookups.
+    // And a DFA that accepts often ends its inputs within a few thousand bytes, about as many as
     // a collapse costs: 4096 inputs of 64 KiB with 0.05% accepting states took 4.6 ms cut and
     // 2.5 ms whole
-    if (d.entry_bytes != 2 || d.num_states > 32768 || !(d.flags & GBFSM_DFA_RARE_ACCEPT))
+    if (d.entry_bytes != 2 || d.num_states > 32768 || !(d.flags & GBFSM_DFA_COLLAPSES) ||
+        !(d.flags & GBFSM_DFA_RARE_ACCEPT))
         return false;
     const uint32_t words = ((uint32_t)d.num_states + 31u) >> 5;
     for (int warps = kSplitMaxWarps; warps >= 1; warps /= 2) {

@@ -15,6 +15,8 @@ in the top bit, plus packed accept bits.
 
 from __future__ import annotations
 
+from functools import lru_cache
+
 import numpy as np
 import torch
 
@@ -451,6 +453,44 @@ class DeviceNFA:
                 + self.eps_edges.numel() + self.accept_words.numel())
 
 
+# the chunked walks of a DFA follow its set of all states until it has this many members
+DFA_ENTRY_STATES = 16  # kEntries (csrc/dfa_chunks.cuh)
+# a set that has not shrunk so far after this many times a random DFA's lookups does not
+COLLAPSE_SCHEDULES = 8
+# how much slower than a random DFA's it may shrink for a plain launch to cut its inputs:
+# 4096 inputs of 64 KiB on 4096 random states spend 3 of 7.4 ms on it, and whole take 12.6
+SPLIT_SCHEDULES = 2
+
+
+@lru_cache(maxsize=1)
+def _trial_texts() -> dict[str, np.ndarray]:
+    """Texts on which a DFA's set of all states is tried: any bytes, lines of printable
+    ones, and digits (a counter over digits leaves every other byte to a sink, so that on
+    any other text its states fall together at once)."""
+    rng = np.random.default_rng(20)
+    n = 1 << 17
+    lines = rng.integers(32, 127, n, dtype=np.uint8)
+    lines[rng.random(n) < 1 / 64] = 10
+    return {"bytes": rng.integers(0, 256, n, dtype=np.uint8), "lines": lines,
+            "digits": rng.integers(48, 58, n, dtype=np.uint8)}
+
+
+def collapse_trial(dfa, schedules: int = COLLAPSE_SCHEDULES) -> dict[str, tuple[int, float, int]]:
+    """For each trial text, the bytes after which ``dfa``'s set of all states has at most
+    DFA_ENTRY_STATES members (-1: not within ``schedules`` times the lookups that a random
+    DFA's takes, or the text), the lookups as a multiple of a random DFA's, and the lookups."""
+    trans = np.ascontiguousarray(dfa.trans, dtype=np.int32)
+    out = np.zeros(3, dtype=np.int64)
+    found = {}
+    for name, text in _trial_texts().items():
+        st = native.lib().gbfsm_dfa_collapse_trial(
+            int(dfa.num_states), trans.ctypes.data, text.ctypes.data, text.size,
+            DFA_ENTRY_STATES, schedules, out.ctypes.data)
+        native.check(st, "gbfsm_dfa_collapse_trial")
+        found[name] = (int(out[0]), int(out[1]) / int(out[2]), int(out[1]))
+    return found
+
+
 class DeviceDFA:
     """A DFA (ours or gpufsm's) resident on a GPU as a packed transition table."""
 
@@ -500,6 +540,15 @@ class DeviceDFA:
         d.entry_bytes = entry_bytes
         rare = self.accept_share is not None and self.accept_share * 50000 <= 1.0
         d.flags = native.DFA_RARE_ACCEPT if rare else 0
+        # how its set of all states shrinks, for the same paths. Digits decide about the plain
+        # launch's cut alone: it gains a factor of two at most and has no longer chunks to
+        # fall back on
+        trial = collapse_trial(dfa) if entry_bytes == 2 else {}
+        if trial and all(t >= 0 and x <= SPLIT_SCHEDULES for t, x, _ in trial.values()):
+            d.flags |= native.DFA_COLLAPSES
+        texts = [trial[k] for k in ("bytes", "lines")] if trial else []
+        if texts and all(t >= 0 for t, _, _ in texts):
+            d.collapse_lookups = max(1, max(n for _, _, n in texts))
         d.table = self.table.data_ptr()
         d.accept_bits = self.accept_bits.data_ptr()
         d.table_bytes = self.table_bytes

@@ -32,7 +32,7 @@ EDGE_SYMBOL_MASK = 0x1FF
 EDGE_ACCEPT = 1 << 9
 EDGE_HAS_EPS = 1 << 10
 CODE_SET = 1 << 11  # GBFSM_CODE_SET
-DFA_RARE_ACCEPT = 1  # GBFSM_DFA_RARE_ACCEPT
+DFA_RARE_ACCEPT, DFA_COLLAPSES = 1, 2  # GBFSM_DFA_*
 
 FLAG_TIMEOUT = -1
 
@@ -100,6 +100,8 @@ class DfaDev(ctypes.Structure):
         ("table", ctypes.c_void_p),
         ("accept_bits", ctypes.c_void_p),
         ("table_bytes", ctypes.c_uint64),
+        ("collapse_lookups", ctypes.c_uint32),
+        ("reserved", ctypes.c_uint32),
     ]
 
 
@@ -233,6 +235,7 @@ SIGNATURES: dict[str, tuple] = {
                                             _vp, _vp]),
     "gbfsm_slots_build": (_i32, [_i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _i64, _vp,
                                  _vp]),
+    "gbfsm_dfa_collapse_trial": (_i32, [_i32, _vp, _vp, _i64, _i32, _i32, _vp]),
     "gbfsm_lanes_stage_limit": (_i32, []),
     "gbfsm_sym_fixup_run": (ctypes.c_int, [_vp, _i32, _i32, _vp, _i32, _vp, _vp, _vp,
                                            _P(ChunkIO), _P(Plan), _vp, _vp, _vp, _vp]),
@@ -256,7 +259,7 @@ SIGNATURES: dict[str, tuple] = {
                                                  _vp]),
 }
 
-ABI_VERSION = 4
+ABI_VERSION = 5
 
 _lib: ctypes.CDLL | None = None
 

@@ -37,7 +37,7 @@
 extern "C" {
 #endif
 
-#define GBFSM_ABI_VERSION 4
+#define GBFSM_ABI_VERSION 5
 #define GBFSM_ANY_SYMBOL 256 /* src/gpufsm/core/nfa.py:16 */
 #define GBFSM_WORD_BITS 64   /* src/gpufsm/core/packing.py:21 */
 
@@ -168,11 +168,18 @@ typedef struct gbfsm_dfa_dev {
     const void *table;
     const uint32_t *accept_bits;
     uint64_t table_bytes;
+    uint32_t collapse_lookups; /* lookups of gbfsm_dfa_collapse_trial over texts of its
+                                  alphabet; 0 = unknown (chunk walks then allow a collapse
+                                  what a random DFA's takes) */
+    uint32_t reserved;
 } gbfsm_dfa_dev;
 
 /* At most one table entry in 50000 leads to an accepting state: a run over uniform bytes
  * goes on for tens of thousands (a hint for how to launch; results do not depend on it). */
 #define GBFSM_DFA_RARE_ACCEPT 1
+/* The set of all states shrinks as fast as a random DFA's on every text tried (a hint like
+ * the last one). */
+#define GBFSM_DFA_COLLAPSES 2
 
 /* How to run a batch. Zero fields select the defaults. */
 typedef struct gbfsm_plan {
@@ -433,6 +440,14 @@ int32_t gbfsm_slots_build(int32_t num_states, const int32_t *sym_row_ptr,
                           const uint8_t *accept, int64_t cap_slots, uint32_t *slots,
                           int64_t cap_pairs, uint32_t *pairs, int64_t cap_codes,
                           uint32_t *codes, int64_t *info);
+
+/* Follow the set of all states of a DFA (HOST int32 [n * 256]) over `text` until it has at
+ * most `want` members (host only; csrc/dfa_trial.cu). out[0] receives the bytes that took,
+ * -1 when the text ended first or `schedules` times the lookups of a random DFA of as many
+ * states were not enough; out[1] the table lookups made, out[2] a random DFA's (want 16).
+ * No counterpart in the reference. */
+int32_t gbfsm_dfa_collapse_trial(int32_t num_states, const int32_t *trans, const uint8_t *text,
+                                 int64_t len, int32_t want, int32_t schedules, int64_t *out);
 
 /* Largest gbfsm_chunk_io.lane_stage_bytes of the lane launch on the current device. */
 int32_t gbfsm_lanes_stage_limit(void);

@@ -1,0 +1,76 @@
+"""Trials of how a DFA's set of all states shrinks (csrc/dfa_trial.cu), on the CPU, against
+the set walk written out."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from abstraction_regret_gb300 import device as D
+from abstraction_regret_gb300 import native
+from abstraction_regret_gb300.automata import DFA, random_dfa
+
+
+def _dfa(trans):
+    n = trans.shape[0]
+    return DFA(num_states=n, start_state=0, accept=np.zeros(n, bool),
+               trans=trans.reshape(-1).astype(np.int32))
+
+
+def _permuting(n, seed=1, alphabet=range(256)):
+    """Bytes of the alphabet permute the states, the others lead to state 0."""
+    rng = np.random.default_rng(seed)
+    trans = np.zeros((n, 256), dtype=np.int32)
+    for c in alphabet:
+        trans[:, c] = rng.permutation(n)
+    return _dfa(trans)
+
+
+@pytest.mark.parametrize("states", [1, 2, 16, 17, 33, 300, 2500])
+def test_trial_is_the_set_walk(states):
+    dfa = random_dfa(states, accept_prob=0.0, seed=states)
+    trans = dfa.trans.reshape(states, 256)
+    for name, text in D._trial_texts().items():
+        members, lookups, pos = np.arange(states), 0, 0
+        while members.size > D.DFA_ENTRY_STATES:
+            lookups += members.size
+            members = np.unique(trans[members, text[pos]])
+            pos += 1
+        got = D.collapse_trial(dfa)[name]
+        assert (got[0], got[2]) == (pos, lookups)
+
+
+@pytest.mark.parametrize("states", [300, 4096, 32768])
+def test_random_dfas_shrink_on_schedule(states):
+    for t, x, _ in D.collapse_trial(random_dfa(states, accept_prob=0.0, seed=3)).values():
+        assert states / 16 < t < states / 4 and 0.5 < x < 1.5
+
+
+def test_permuted_states_never_shrink():
+    trial = D.collapse_trial(_permuting(4096))
+    assert all(t == -1 for t, _, _ in trial.values())
+    # given up after the lookups allowed and at most one step more
+    assert all(x <= D.COLLAPSE_SCHEDULES + 1 for _, x, _ in trial.values())
+    digits = D.collapse_trial(_permuting(4096, alphabet=range(48, 58)))
+    assert digits["bytes"][0] <= 3 and digits["lines"][0] <= 16 and digits["digits"][0] == -1
+
+
+def test_a_set_that_stops_above_the_entry_states():
+    trans = np.random.default_rng(4).integers(0, 17, size=(200, 256))
+    for c in range(256):
+        trans[:17, c] = np.random.default_rng(c).permutation(17)
+    assert all(t == -1 for t, _, _ in D.collapse_trial(_dfa(trans)).values())
+    trans = trans % 16
+    for c in range(256):
+        trans[:16, c] = np.random.default_rng(c).permutation(16)
+    assert all(t == 1 for t, _, _ in D.collapse_trial(_dfa(trans)).values())
+
+
+def test_bad_tables_are_refused():
+    dfa = _permuting(20)
+    dfa.trans[:] = 20
+    with pytest.raises(ValueError):
+        D.collapse_trial(dfa)
+    lib, out = native.lib(), np.zeros(3, np.int64)
+    assert lib.gbfsm_dfa_collapse_trial(0, None, None, 0, 16, 8, out.ctypes.data) == \
+        native.INVALID_ARG

@@ -142,3 +142,68 @@ def test_every_alignment_and_tail(states):
     flags = _plain(dfa, inputs)
     assert 0 < int(flags.sum()) < len(inputs)
     _check(dfa, inputs)
+
+
+def _permuting(n, seed, alphabet):
+    """Bytes of the alphabet permute the states, the others lead to state 0; state n - 1
+    accepts and is entered from state 1 by byte 48 alone."""
+    rng = np.random.default_rng(seed)
+    trans = np.zeros((n, 256), dtype=np.int32)
+    for c in alphabet:
+        trans[:n - 1, c] = rng.permutation(n - 1)
+    trans[1, 48] = n - 1
+    return DFA(num_states=n, start_state=0, accept=np.arange(n) == n - 1,
+               trans=trans.reshape(-1))
+
+
+def _ms(call, repeats=3):
+    import torch
+
+    best = float("inf")
+    for _ in range(1 + repeats):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        call()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+@pytest.mark.parametrize("alphabet", [range(256), range(48, 58)])
+def test_plain_launch_of_permuted_states(alphabet):
+    """A cut would follow all states through every chunk: the launch takes no longer than
+    the serial walk of its longest input (under 0.3 us a byte) allows."""
+    import torch
+
+    from abstraction_regret_gb300.executors import CudaDFAExecutor
+
+    dfa = _permuting(4096, 7, alphabet)
+    rng = np.random.default_rng(8)
+    inputs = [rng.integers(48, 58, n, dtype=np.uint8).tobytes()
+              for n in [16384] * 60 + [0, 100, 5000, 9999]]
+    _plain(dfa, inputs)
+    ex = CudaDFAExecutor(dfa)
+    data, off = O.flatten(inputs)
+    d = torch.from_numpy(np.concatenate([data, np.zeros(16, np.uint8)])).cuda()
+    o = torch.from_numpy(off).cuda()
+    out = torch.zeros((3, len(inputs)), dtype=torch.int32, device="cuda")
+    ms = _ms(lambda: ex.launch(d, o, len(inputs), out[0], out[1], out[2]))
+    assert ms < 16384 * 0.3e-3 * 2
+
+
+@pytest.mark.parametrize("alphabet", [range(256), range(48, 58)])
+def test_chunks_of_permuted_states(alphabet):
+    """Chunks give up on a set that does not shrink: verdicts are exact and the step takes no
+    longer than the serial walk of its longest input allows."""
+    from abstraction_regret_gb300.engine import GraphRunner
+
+    dfa = _permuting(4096, 9, alphabet)
+    rng = np.random.default_rng(10)
+    inputs = [rng.integers(48, 58, n, dtype=np.uint8).tobytes()
+              for n in [16384] * 60 + [0, 100, 5000, 9999]]
+    _check(dfa, inputs, dfa_chunk_bytes=4096)
+    eng = PersistentEngine([dfa], dfa_chunk_bytes=4096)
+    data, off = O.flatten(inputs)
+    runner = GraphRunner(eng, [0] * len(inputs), data, off)
+    assert _ms(runner.kernel_only) < 16384 * 0.3e-3 * 2
