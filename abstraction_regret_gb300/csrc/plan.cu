@@ -43,9 +43,6 @@ constexpr int kPlanThreads = 1024;
 constexpr int kBuckets = 64;  // (two per lane of the warp that lays them out)
 constexpr int kLaneGroup = 32;
 constexpr int64_t kMaxChunk = 1 << 20;
-// L2 gather rate x time of a dependent lookup / lookups of a collapse per byte of the
-// shortest chunk (150 G/s x 0.2 us / 50): see the DFA chunk length
-constexpr double kDfaBalance = 600.0;
 
 // per-input scratch (int32 arrays of n entries) and per-bucket tables
 struct PlanScratch {
@@ -234,14 +231,14 @@ __global__ void __launch_bounds__(kPlanThreads) plan_scan_kernel(gbfsm_batch_pla
     // A chunk costs the walk of its set of all states, about 50 m table lookups at the L2's
     // gather rate R for the whole batch, and its own length L in dependent lookups of t
     // each: the sum of B / L * 50 m / R and L t is least at L = sqrt(B m 50 / (R t)), with
-    // 50 / (R t) = 1 / kDfaBalance. And at most one wave of chunks: rounding each input up
+    // 50 / (R t) = 1 / GBFSM_PLAN_DFA_BALANCE. And at most one wave of chunks: rounding each input up
     // to whole chunks adds at most one per input, so B / (chunks at a time - inputs).
     int64_t dfa_target = 0;
     bool dfa_split = false;
     if (a.dfa_warps > 0 && dfa_bytes > 0) {
         const int64_t w = a.dfa_warps > dfa_long ? a.dfa_warps - dfa_long : 1;
         dfa_target = (dfa_bytes + w - 1) / w;
-        const int64_t balanced = (int64_t)sqrt((double)dfa_work / kDfaBalance);
+        const int64_t balanced = (int64_t)sqrt((double)dfa_work / GBFSM_PLAN_DFA_BALANCE);
         if (balanced > dfa_target) dfa_target = balanced;
         dfa_target = (dfa_target + 63) / 64 * 64;
         if (dfa_target > (int64_t)1 << 30) dfa_target = (int64_t)1 << 30;

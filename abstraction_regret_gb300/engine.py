@@ -71,7 +71,6 @@ DFA_CHUNK_MAX_STATES = 32768
 DFA_CHUNK_MIN = 1024
 DFA_CHUNK_FLOOR = 1024  # the shortest DFA chunk a caller may ask for
 DFA_CHUNK_STATES = 4
-DFA_CHUNK_BALANCE = 600.0  # kDfaBalance (csrc/plan.cu)
 # the most a DFA chunk's walk continues past its end, as a share of the shortest chunk; 1 or
 # more: no limit but the next entry position
 DFA_OVERLAP_CHUNKS = 1.0
@@ -269,7 +268,7 @@ class DevicePlan:
         c = engine.min_dfa_chunk
         fixups = min(int(n), int(total_bytes) // (2 * c)) + 1
         if engine.dfa_warps > 0:
-            length = max(c, int(math.sqrt(int(total_bytes) * c / DFA_CHUNK_BALANCE)))
+            length = max(c, int(math.sqrt(int(total_bytes) * c / native.PLAN_DFA_BALANCE)))
             return 3 * int(total_bytes) // length + 2, fixups
         return 3 * int(total_bytes) // (2 * c) + 2, fixups
 

@@ -148,6 +148,7 @@ class ChunkIO(ctypes.Structure):
 
 LANE_STAGE_NONE, LANE_STAGE_WIDE, LANE_STAGE_NARROW = range(3)  # GBFSM_LANE_STAGE_*
 
+PLAN_DFA_BALANCE = 600  # GBFSM_PLAN_DFA_BALANCE
 PLAN_MAX_SLICES = 16  # GBFSM_PLAN_MAX_SLICES
 
 

@@ -533,6 +533,10 @@ gbfsm_status gbfsm_lanes_run_range(const gbfsm_automaton *table, int32_t n_autom
                                          minimum (0: from aut_dfa_chunk alone) */
 #define GBFSM_PLAN_SLICES 16       /* {first, count} LANES task range of slice k at
                                       16 + 2k, for gbfsm_lanes_run_range */
+/* The planner's DFA chunk length (csrc/plan.cu) is sqrt(bytes x shortest chunk / this): the
+ * L2's gather rate x the time of a dependent lookup / a collapse's lookups per byte of the
+ * shortest chunk (150 G/s x 0.2 us / 50). Callers size the chunk buffers by it. */
+#define GBFSM_PLAN_DFA_BALANCE 600
 #define GBFSM_PLAN_MAX_SLICES 16
 
 typedef struct gbfsm_batch_plan_args {
