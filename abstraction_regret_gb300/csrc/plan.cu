@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kPlanThreads) plan_scan_kernel(gbfsm_batch_pla
             if (m > 0 && r.len >= 2 * m) {
                 dfa_bytes += r.len;
                 dfa_long += 1;
-                dfa_work += r.len * m;
+                dfa_work += r.len * (a.aut_dfa_cost ? (int64_t)a.aut_dfa_cost[r.aut] : 50 * m);
             }
         }
     }
@@ -227,12 +227,12 @@ __global__ void __launch_bounds__(kPlanThreads) plan_scan_kernel(gbfsm_batch_pla
         dfa_long = t5[3];
         dfa_work = t5[4];
     }
-    // The batch's DFA chunk length (before each DFA's minimum m, a quarter of its states).
-    // A chunk costs the walk of its set of all states, about 50 m table lookups at the L2's
-    // gather rate R for the whole batch, and its own length L in dependent lookups of t
-    // each: the sum of B / L * 50 m / R and L t is least at L = sqrt(B m 50 / (R t)), with
-    // 50 / (R t) = 1 / GBFSM_PLAN_DFA_BALANCE. And at most one wave of chunks: rounding each input up
-    // to whole chunks adds at most one per input, so B / (chunks at a time - inputs).
+    // The batch's DFA chunk length (before each DFA's minimum). A chunk costs the walk of
+    // its set of all states, c table lookups at the L2's gather rate R for the whole batch,
+    // and its own length L in dependent lookups of t each: the sum of B / L * c / R and L t
+    // is least at L = sqrt(B c / (R t)), with R t = GBFSM_PLAN_DFA_BALANCE. And at most one
+    // wave of chunks: rounding each input up to whole chunks adds at most one per input, so
+    // B / (chunks at a time - inputs).
     int64_t dfa_target = 0;
     bool dfa_split = false;
     if (a.dfa_warps > 0 && dfa_bytes > 0) {

@@ -467,12 +467,10 @@ def _trial_texts() -> dict[str, np.ndarray]:
     """Texts on which a DFA's set of all states is tried: any bytes, lines of printable
     ones, and digits (a counter over digits leaves every other byte to a sink, so that on
     any other text its states fall together at once)."""
-    rng = np.random.default_rng(20)
-    n = 1 << 17
-    lines = rng.integers(32, 127, n, dtype=np.uint8)
-    lines[rng.random(n) < 1 / 64] = 10
-    return {"bytes": rng.integers(0, 256, n, dtype=np.uint8), "lines": lines,
-            "digits": rng.integers(48, 58, n, dtype=np.uint8)}
+    any_byte, a, b = np.frombuffer(np.random.default_rng(20).bytes(3 << 15),
+                                   dtype=np.uint8).reshape(3, -1)
+    line = np.concatenate([32 + np.arange(252) % 95, [10] * 4]).astype(np.uint8)
+    return {"bytes": any_byte, "lines": line[a], "digits": (48 + b % 10).astype(np.uint8)}
 
 
 def collapse_trial(dfa, schedules: int = COLLAPSE_SCHEDULES) -> dict[str, tuple[int, float, int]]:
@@ -547,8 +545,11 @@ class DeviceDFA:
         if trial and all(t >= 0 and x <= SPLIT_SCHEDULES for t, x, _ in trial.values()):
             d.flags |= native.DFA_COLLAPSES
         texts = [trial[k] for k in ("bytes", "lines")] if trial else []
+        # bytes and lookups of a chunk's collapse (no bytes: it does not end)
+        self.collapse_bytes, self.collapse_lookups = None, max([k for _, _, k in texts] or [0])
         if texts and all(t >= 0 for t, _, _ in texts):
-            d.collapse_lookups = max(1, max(n for _, _, n in texts))
+            self.collapse_bytes = max(t for t, _, _ in texts)
+            d.collapse_lookups = max(1, self.collapse_lookups)
         d.table = self.table.data_ptr()
         d.accept_bits = self.accept_bits.data_ptr()
         d.table_bytes = self.table_bytes

@@ -64,13 +64,19 @@ LANE_WARPS_PER_SM = 32
 # DFA chunking (csrc/dfa_chunks.cu): the largest DFA whose inputs are chunked (2-byte
 # table entries), and the shortest DFA chunk: at least DFA_CHUNK_MIN bytes and a byte per
 # DFA_CHUNK_STATES states. A chunk follows the set of all states until it has 16 members,
-# which takes a random DFA about n / 8 bytes; twice that leaves room for slower ones (a
-# chunk that ends before is walked through by the one before it). The planner lengthens the
-# chunks of larger batches.
+# which takes a random DFA about n / 8 bytes and others as long as a trial of them says
+# (device.collapse_trial); a chunk that ends before is walked through by the one before it,
+# so the shortest one is half as long again. A DFA whose set did not shrink on trial is cut
+# into chunks of at least DFA_CHUNK_LONG bytes and DFA_CHUNK_LONG_STATES bytes a state, and
+# its shorter inputs run whole: 64 inputs of 16 KiB on 4096 permuted states took 34.8 ms in
+# chunks of 1344 bytes and take 3.5 whole. The planner lengthens the chunks of larger batches.
 DFA_CHUNK_MAX_STATES = 32768
 DFA_CHUNK_MIN = 1024
 DFA_CHUNK_FLOOR = 1024  # the shortest DFA chunk a caller may ask for
 DFA_CHUNK_STATES = 4
+DFA_CHUNK_LONG = 16 << 10
+DFA_CHUNK_LONG_STATES = 8
+DFA_COLLAPSE_PER_BYTE = 50  # lookups of a random DFA's collapse / its shortest chunk
 # the most a DFA chunk's walk continues past its end, as a share of the shortest chunk; 1 or
 # more: no limit but the next entry position
 DFA_OVERLAP_CHUNKS = 1.0
@@ -86,9 +92,22 @@ PIPELINE_LANE_WAVES = 2
 
 
 def dfa_chunk_length(num_states: int) -> int:
-    """Shortest chunk for the long inputs of a DFA of ``num_states`` states (a multiple of
-    64 bytes); an input is chunked when it holds two chunks."""
+    """Shortest chunk for the long inputs of a random DFA of ``num_states`` states (a
+    multiple of 64 bytes); an input is chunked when it holds two chunks."""
     return -(-max(DFA_CHUNK_MIN, int(num_states) // DFA_CHUNK_STATES) // 64) * 64
+
+
+def dfa_chunk_plan(num_states: int, collapse_bytes: int | None, collapse_lookups: int
+                   ) -> tuple[int, int]:
+    """``(shortest chunk in bytes, lookups of its collapse)`` of a DFA whose set of all
+    states took ``collapse_bytes`` (None: never) and ``collapse_lookups`` on trial."""
+    n = int(num_states)
+    random = dfa_chunk_length(n)
+    longest = -(-max(DFA_CHUNK_LONG, DFA_CHUNK_LONG_STATES * n) // 64) * 64
+    cost = max(DFA_COLLAPSE_PER_BYTE * random, int(collapse_lookups))
+    if collapse_bytes is None:
+        return longest, cost
+    return min(longest, max(random, -(-3 * int(collapse_bytes) // 128) * 64)), cost
 
 
 def dfa_overlap_bytes(chunk_length: int) -> int:
@@ -268,7 +287,8 @@ class DevicePlan:
         c = engine.min_dfa_chunk
         fixups = min(int(n), int(total_bytes) // (2 * c)) + 1
         if engine.dfa_warps > 0:
-            length = max(c, int(math.sqrt(int(total_bytes) * c / native.PLAN_DFA_BALANCE)))
+            length = max(c, int(math.sqrt(int(total_bytes) * engine.min_dfa_cost
+                                          / native.PLAN_DFA_BALANCE)))
             return 3 * int(total_bytes) // length + 2, fixups
         return 3 * int(total_bytes) // (2 * c) + 2, fixups
 
@@ -309,6 +329,7 @@ class DevicePlan:
         a.aut_class = eng.aut_class.data_ptr()
         if eng.aut_dfa_chunk is not None:
             a.aut_dfa_chunk = eng.aut_dfa_chunk.data_ptr()
+            a.aut_dfa_cost = eng.aut_dfa_cost.data_ptr()
             a.tasks_dfa_chunk = self.tasks_dfa_chunk
             a.tasks_dfa_fixup = self.tasks_dfa_fixup
             a.dfa_latch = self.dfa_latch.data_ptr()
@@ -483,7 +504,7 @@ class PersistentEngine:
                  resident=None, dfa_chunk_bytes: int | None = None) -> None:
         """``chunk_bytes``: 0 = chosen per batch, None = never chunk, else a fixed size.
         ``dfa_chunk_bytes``: chunk length of long DFA inputs; None = from each DFA's size
-        (dfa_chunk_length()), 0 = DFA inputs always run whole, else this length (rounded up
+        and its trial (dfa_chunk_plan()), 0 = DFA inputs always run whole, else this length (rounded up
         to 64 bytes, at least DFA_CHUNK_FLOOR) for every DFA.
         ``lane_pair_mean``: largest mean two-byte superset for one-lane-per-chunk tasks.
         ``resident``: device layouts already built for ``automata`` (DeviceNFA /
@@ -526,13 +547,16 @@ class PersistentEngine:
             self.workspace = torch.zeros(self.ws_bytes, dtype=torch.uint8, device=self.device)
             # long DFA inputs are cut into chunks walked in parallel (DFA_CHUNK tasks)
             dfa_chunk = [0] * len(self.automata)
+            dfa_cost = [0] * len(self.automata)
             if chunk_bytes is not None and dfa_chunk_bytes != 0:
                 for i, (d, k) in enumerate(zip(self.dev, self.kinds)):
                     if k is Kind.DFA and d.entry_bytes == 2 and \
                             d.num_states <= DFA_CHUNK_MAX_STATES:
-                        dfa_chunk[i] = (dfa_chunk_length(d.num_states) if dfa_chunk_bytes is None
-                                        else -(-max(DFA_CHUNK_FLOOR, int(dfa_chunk_bytes))
-                                               // 64) * 64)
+                        dfa_chunk[i], dfa_cost[i] = dfa_chunk_plan(
+                            d.num_states, d.collapse_bytes, d.collapse_lookups)
+                        if dfa_chunk_bytes is not None:
+                            dfa_chunk[i] = -(-max(DFA_CHUNK_FLOOR, int(dfa_chunk_bytes))
+                                             // 64) * 64
             self.dfa_chunk = dfa_chunk
             self.dfa_max_states = max([d.num_states for d, c in zip(self.dev, dfa_chunk) if c]
                                       or [0])
@@ -587,7 +611,10 @@ class PersistentEngine:
         self.min_chunk = MIN_CHUNK_SMALL_STARTS if small_starts else MIN_CHUNK
         self.aut_dfa_chunk = (torch.tensor(self.dfa_chunk, dtype=torch.int32, device=self.device)
                               if any(self.dfa_chunk) else None)
+        self.aut_dfa_cost = (torch.tensor(dfa_cost, dtype=torch.int32, device=self.device)
+                             if any(self.dfa_chunk) else None)
         self.min_dfa_chunk = min([c for c in self.dfa_chunk if c] or [0])
+        self.min_dfa_cost = min([c for c, m in zip(dfa_cost, self.dfa_chunk) if m] or [0])
         # chunk lengths follow the batch (one wave of the chunk launch) unless fixed
         self.dfa_warps = 0
         if self.aut_dfa_chunk is not None and dfa_chunk_bytes is None:

@@ -148,7 +148,7 @@ class ChunkIO(ctypes.Structure):
 
 LANE_STAGE_NONE, LANE_STAGE_WIDE, LANE_STAGE_NARROW = range(3)  # GBFSM_LANE_STAGE_*
 
-PLAN_DFA_BALANCE = 600  # GBFSM_PLAN_DFA_BALANCE
+PLAN_DFA_BALANCE = 30000  # GBFSM_PLAN_DFA_BALANCE
 PLAN_MAX_SLICES = 16  # GBFSM_PLAN_MAX_SLICES
 
 
@@ -158,6 +158,7 @@ class BatchPlanArgs(ctypes.Structure):
         ("offsets", ctypes.c_void_p), ("ends", ctypes.c_void_p),
         ("aut_ids", ctypes.c_void_p), ("aut_class", ctypes.c_void_p),
         ("aut_dfa_chunk", ctypes.c_void_p),
+        ("aut_dfa_cost", ctypes.c_void_p),
         ("lane_warps", ctypes.c_int32), ("persist_warps", ctypes.c_int32),
         ("dfa_warps", ctypes.c_int32),
         ("min_chunk", ctypes.c_int32), ("fixed_chunk", ctypes.c_int32),

@@ -533,10 +533,10 @@ gbfsm_status gbfsm_lanes_run_range(const gbfsm_automaton *table, int32_t n_autom
                                          minimum (0: from aut_dfa_chunk alone) */
 #define GBFSM_PLAN_SLICES 16       /* {first, count} LANES task range of slice k at
                                       16 + 2k, for gbfsm_lanes_run_range */
-/* The planner's DFA chunk length (csrc/plan.cu) is sqrt(bytes x shortest chunk / this): the
- * L2's gather rate x the time of a dependent lookup / a collapse's lookups per byte of the
- * shortest chunk (150 G/s x 0.2 us / 50). Callers size the chunk buffers by it. */
-#define GBFSM_PLAN_DFA_BALANCE 600
+/* The planner's DFA chunk length (csrc/plan.cu) is sqrt(bytes x a collapse's lookups / this):
+ * the L2's gather rate x the time of a dependent lookup (150 G/s x 0.2 us). Callers size the
+ * chunk buffers by it. */
+#define GBFSM_PLAN_DFA_BALANCE 30000
 #define GBFSM_PLAN_MAX_SLICES 16
 
 typedef struct gbfsm_batch_plan_args {
@@ -549,6 +549,8 @@ typedef struct gbfsm_batch_plan_args {
     const int32_t *aut_class; /* device [n_automata]: GBFSM_PLAN_* */
     const int32_t *aut_dfa_chunk; /* device [n_automata] or NULL: shortest DFA chunk of each
                                      automaton, bytes (0 = run the DFA's inputs whole) */
+    const int32_t *aut_dfa_cost;  /* device [n_automata] or NULL (50 for each byte of the
+                                     shortest chunk): table lookups of a chunk's collapse */
     int32_t lane_warps;       /* resident warps of the lane launch (SMs x
                                  gbfsm_lanes_warps_per_sm) */
     int32_t persist_warps;    /* resident warps of the persistent launch */
@@ -556,7 +558,7 @@ typedef struct gbfsm_batch_plan_args {
                                  gbfsm_dfa_chunks_warps_per_sm), or 0. An input of DFA a is
                                  cut into chunks of max(aut_dfa_chunk[a], L) bytes when it
                                  holds two of them; L balances the cost of a chunk's
-                                 collapse (its minimum's share) against its walk over the
+                                 collapse (aut_dfa_cost) against its walk over the
                                  batch's DFA inputs that hold two chunks of their own
                                  minimum, at most dfa_warps chunks (csrc/plan.cu) */
     int32_t min_chunk;        /* shortest chunk (bytes) */

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from abstraction_regret_gb300 import device as D
+from abstraction_regret_gb300 import engine as E
 from abstraction_regret_gb300 import native
 from abstraction_regret_gb300.automata import DFA, random_dfa
 
@@ -74,3 +75,46 @@ def test_bad_tables_are_refused():
     lib, out = native.lib(), np.zeros(3, np.int64)
     assert lib.gbfsm_dfa_collapse_trial(0, None, None, 0, 16, 8, out.ctypes.data) == \
         native.INVALID_ARG
+
+
+def _lazy(n, share, seed=1):
+    """Every byte permutes the states but for a share of them, which it sends anywhere: the
+    set of all states shrinks more slowly than a random DFA's the smaller the share."""
+    rng = np.random.default_rng(seed)
+    trans = np.empty((n, 256), dtype=np.int32)
+    for c in range(256):
+        p = rng.permutation(n)
+        anywhere = rng.random(n) < share
+        p[anywhere] = rng.integers(0, n, int(anywhere.sum()))
+        trans[:, c] = p
+    return _dfa(trans)
+
+
+@pytest.mark.parametrize("states,share,seed", [(4096, 1.0, 1), (16384, 1.0, 2), (16384, 0.3, 3),
+                                               (4096, 0.15, 4), (2000, 0.0, 5)])
+def test_shortest_chunk_holds_the_collapse(states, share, seed):
+    """The shortest chunk is a random DFA's, or half as long again as the collapse where that
+    takes longer, or the long length where the set does not shrink."""
+    dfa = _lazy(states, share, seed)
+    trial = D.collapse_trial(dfa)
+    texts = [trial["bytes"], trial["lines"]]
+    ends = all(t >= 0 for t, _, _ in texts)
+    length, cost = E.dfa_chunk_plan(states, max(t for t, _, _ in texts) if ends else None,
+                                    max(k for _, _, k in texts))
+    assert length % 64 == 0 and cost >= max(k for _, _, k in texts)
+    assert ends == (share > 0.1)
+    if share == 1.0:
+        assert length == E.dfa_chunk_length(states)
+    elif ends:
+        assert E.dfa_chunk_length(states) < length < 8 * states
+        # the collapse of other texts ends within the chunk
+        rng = np.random.default_rng(6)
+        trans = dfa.trans.reshape(states, 256)
+        for _ in range(4):
+            members, pos = np.arange(states), 0
+            while members.size > D.DFA_ENTRY_STATES:
+                members = np.unique(trans[members, int(rng.integers(0, 256))])
+                pos += 1
+            assert pos < length
+    else:
+        assert length == max(16 << 10, 8 * states)

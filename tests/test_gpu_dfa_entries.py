@@ -207,3 +207,43 @@ def test_chunks_of_permuted_states(alphabet):
     data, off = O.flatten(inputs)
     runner = GraphRunner(eng, [0] * len(inputs), data, off)
     assert _ms(runner.kernel_only) < 16384 * 0.3e-3 * 2
+
+
+def test_inputs_of_permuted_states_run_whole():
+    """Inputs shorter than two long chunks are not cut: the step takes no longer than the
+    serial walk of its longest input allows."""
+    from abstraction_regret_gb300.engine import GraphRunner
+
+    dfa = _permuting(4096, 11, range(256))
+    rng = np.random.default_rng(12)
+    inputs = [rng.integers(0, 256, n, dtype=np.uint8).tobytes()
+              for n in [16384] * 60 + [0, 100, 5000, 9999]]
+    _check(dfa, inputs)
+    data, off = O.flatten(inputs)
+    runner = GraphRunner(PersistentEngine([dfa]), [0] * len(inputs), data, off)
+    assert _ms(runner.kernel_only) < 16384 * 0.3e-3 * 2
+
+
+@pytest.mark.parametrize("states,share", [(8192, 0.15), (16384, 0.3), (16384, 1.0)])
+def test_slow_collapses_end_in_their_chunks(states, share):
+    """Bytes permute all states but a share, which they send anywhere: chunks are long enough
+    for the set to shrink, so nearly all of them have entry states."""
+    from abstraction_regret_gb300 import native
+
+    rng = np.random.default_rng(states)
+    trans = np.empty((states, 256), dtype=np.int32)
+    for c in range(256):
+        p = rng.permutation(states)
+        anywhere = rng.random(states) < share
+        p[anywhere] = rng.integers(0, states, int(anywhere.sum()))
+        trans[:, c] = p
+    dfa = DFA(num_states=states, start_state=0, accept=np.zeros(states, bool),
+              trans=trans.reshape(-1))
+    eng = PersistentEngine([dfa])
+    inputs = [rng.integers(0, 256, n, dtype=np.uint8).tobytes() for n in (1 << 20, 300_000)]
+    f, l, e, _, _ = eng.run_requests([0, 0], inputs, with_examined=True)
+    assert not f.any() and e.tolist() == [len(x) for x in inputs]
+    n = int(eng._dplan.h_header.numpy()[native.PLAN_CHUNKS])
+    p = eng._dplan.records[: n * native.CHUNK_RECORD_BYTES].cpu().numpy().view(np.int32) \
+        .reshape(n, -1)[:, 0]
+    assert n >= 8 and (p >= 0).mean() > 0.95
