@@ -456,7 +456,7 @@ class DeviceNFA:
 # the chunked walks of a DFA follow its set of all states until it has this many members
 DFA_ENTRY_STATES = 16  # kEntries (csrc/dfa_chunks.cuh)
 # a set that has not shrunk so far after this many times a random DFA's lookups does not
-COLLAPSE_SCHEDULES = 8
+COLLAPSE_SCHEDULES = 32
 # how much slower than a random DFA's it may shrink for a plain launch to cut its inputs:
 # 4096 inputs of 64 KiB on 4096 random states spend 3 of 7.4 ms on it, and whole take 12.6
 SPLIT_SCHEDULES = 2
@@ -473,19 +473,23 @@ def _trial_texts() -> dict[str, np.ndarray]:
     return {"bytes": any_byte, "lines": line[a], "digits": (48 + b % 10).astype(np.uint8)}
 
 
-def collapse_trial(dfa, schedules: int = COLLAPSE_SCHEDULES) -> dict[str, tuple[int, float, int]]:
+def collapse_trial(dfa) -> dict[str, tuple[int, float, int]]:
     """For each trial text, the bytes after which ``dfa``'s set of all states has at most
-    DFA_ENTRY_STATES members (-1: not within ``schedules`` times the lookups that a random
-    DFA's takes, or the text), the lookups as a multiple of a random DFA's, and the lookups."""
+    DFA_ENTRY_STATES members (-1: not within the text or COLLAPSE_SCHEDULES times the lookups
+    that a random DFA's takes, SPLIT_SCHEDULES times for digits), the lookups as a multiple of
+    a random DFA's, and the lookups. Up to the first text on which it has not."""
     trans = np.ascontiguousarray(dfa.trans, dtype=np.int32)
     out = np.zeros(3, dtype=np.int64)
     found = {}
     for name, text in _trial_texts().items():
         st = native.lib().gbfsm_dfa_collapse_trial(
             int(dfa.num_states), trans.ctypes.data, text.ctypes.data, text.size,
-            DFA_ENTRY_STATES, schedules, out.ctypes.data)
+            DFA_ENTRY_STATES, SPLIT_SCHEDULES if name == "digits" else COLLAPSE_SCHEDULES,
+            out.ctypes.data)
         native.check(st, "gbfsm_dfa_collapse_trial")
         found[name] = (int(out[0]), int(out[1]) / int(out[2]), int(out[1]))
+        if found[name][0] < 0:
+            break
     return found
 
 
@@ -542,9 +546,10 @@ class DeviceDFA:
         # launch's cut alone: it gains a factor of two at most and has no longer chunks to
         # fall back on
         trial = collapse_trial(dfa) if entry_bytes == 2 else {}
-        if trial and all(t >= 0 and x <= SPLIT_SCHEDULES for t, x, _ in trial.values()):
+        if len(trial) == 3 and all(t >= 0 and x <= SPLIT_SCHEDULES
+                                   for t, x, _ in trial.values()):
             d.flags |= native.DFA_COLLAPSES
-        texts = [trial[k] for k in ("bytes", "lines")] if trial else []
+        texts = [trial[k] for k in ("bytes", "lines") if k in trial]
         # bytes and lookups of a chunk's collapse (no bytes: it does not end)
         self.collapse_bytes, self.collapse_lookups = None, max([k for _, _, k in texts] or [0])
         if texts and all(t >= 0 for t, _, _ in texts):
