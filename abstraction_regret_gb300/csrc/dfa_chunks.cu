@@ -49,13 +49,18 @@ __global__ void __launch_bounds__(kDfaChunkThreads, 6) dfa_collapse_kernel(
     uint16_t *list = reinterpret_cast<uint16_t *>(bm1 + words);
     // (a warp per CTA first, so that few tasks spread over the SMs)
     const int nwarps = (int)gridDim.x * kDfaChunkWarps;
-    for (int t = warp_in_cta * (int)gridDim.x + (int)blockIdx.x; t < n_tasks; t += nwarps) {
-        const gbfsm_task task = tasks[t];
+    const int t0 = warp_in_cta * (int)gridDim.x + (int)blockIdx.x;
+    const int rounds = t0 < n_tasks ? (n_tasks - t0 + nwarps - 1) / nwarps : 0;
+    // twice over the tasks, the inputs' first chunks in the first round: an input that accepts
+    // early is then latched before a later wave begins its other chunks
+    for (int r = 0; r < 2 * rounds; ++r) {
+        const gbfsm_task task = tasks[t0 + (r < rounds ? r : r - rounds) * nwarps];
         if (task.kind != GBFSM_TASK_DFA_CHUNK ||
             !dfa_task_ok(task, table, n_automata, chunks, n_chunks, words))
             continue;
-        const gbfsm_dfa_dev d = table[task.automaton].dfa;
         const gbfsm_chunk ch = chunks[task.first];
+        if ((ch.index == 0) != (r < rounds)) continue;
+        const gbfsm_dfa_dev d = table[task.automaton].dfa;
         const int64_t off = offsets[ch.input];
         DfaChunkRecord *rec = dfa_record(records, task.first);
         int32_t *lt = latch ? latch + ch.input : nullptr;

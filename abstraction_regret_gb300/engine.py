@@ -69,13 +69,19 @@ LANE_WARPS_PER_SM = 32
 # so the shortest one is half as long again. A DFA whose set did not shrink on trial is cut
 # into chunks of at least DFA_CHUNK_LONG bytes and DFA_CHUNK_LONG_STATES bytes a state, and
 # its shorter inputs run whole: 64 inputs of 16 KiB on 4096 permuted states took 34.8 ms in
-# chunks of 1344 bytes and take 3.5 whole. The planner lengthens the chunks of larger batches.
+# chunks of 1344 bytes and take 3.5 whole. So is a DFA that accepts every
+# DFA_OFTEN_BYTES bytes on average, whose inputs all but end within the 4096 bytes that their
+# first chunk walks before anything else: the other chunks' collapses are for nothing (0.5% of
+# the entries accepting, 300 inputs of up to 4 MiB 1.13 ms in short chunks, 0.75 in long ones;
+# 0.2% 2.7 and 1.9; at 0.08% the inputs that then run whole cost more than that saves). The
+# planner lengthens the chunks of larger batches.
 DFA_CHUNK_MAX_STATES = 32768
 DFA_CHUNK_MIN = 1024
 DFA_CHUNK_FLOOR = 1024  # the shortest DFA chunk a caller may ask for
 DFA_CHUNK_STATES = 4
 DFA_CHUNK_LONG = 16 << 10
 DFA_CHUNK_LONG_STATES = 8
+DFA_OFTEN_BYTES = 700
 DFA_COLLAPSE_PER_BYTE = 50  # lookups of a random DFA's collapse / its shortest chunk
 # the most a DFA chunk's walk continues past its end, as a share of the shortest chunk; 1 or
 # more: no limit but the next entry position
@@ -97,15 +103,17 @@ def dfa_chunk_length(num_states: int) -> int:
     return -(-max(DFA_CHUNK_MIN, int(num_states) // DFA_CHUNK_STATES) // 64) * 64
 
 
-def dfa_chunk_plan(num_states: int, collapse_bytes: int | None, collapse_lookups: int
-                   ) -> tuple[int, int]:
+def dfa_chunk_plan(num_states: int, collapse_bytes: int | None, collapse_lookups: int,
+                   accept_share: float = 0.0) -> tuple[int, int]:
     """``(shortest chunk in bytes, lookups of its collapse)`` of a DFA whose set of all
-    states took ``collapse_bytes`` (None: never) and ``collapse_lookups`` on trial."""
+    states took ``collapse_bytes`` (None: never) and ``collapse_lookups`` on trial and
+    ``accept_share`` of whose table entries lead to accepting states."""
     n = int(num_states)
     random = dfa_chunk_length(n)
     longest = -(-max(DFA_CHUNK_LONG, DFA_CHUNK_LONG_STATES * n) // 64) * 64
-    cost = max(DFA_COLLAPSE_PER_BYTE * random, int(collapse_lookups))
-    if collapse_bytes is None:
+    # (a random DFA's lookups are up to a quarter more than the rate that it was balanced at)
+    cost = max(DFA_COLLAPSE_PER_BYTE * random, int(collapse_lookups / 1.25))
+    if collapse_bytes is None or accept_share * DFA_OFTEN_BYTES >= 1.0:
         return longest, cost
     return min(longest, max(random, -(-3 * int(collapse_bytes) // 128) * 64)), cost
 
@@ -553,7 +561,8 @@ class PersistentEngine:
                     if k is Kind.DFA and d.entry_bytes == 2 and \
                             d.num_states <= DFA_CHUNK_MAX_STATES:
                         dfa_chunk[i], dfa_cost[i] = dfa_chunk_plan(
-                            d.num_states, d.collapse_bytes, d.collapse_lookups)
+                            d.num_states, d.collapse_bytes, d.collapse_lookups,
+                            d.accept_share)
                         if dfa_chunk_bytes is not None:
                             dfa_chunk[i] = -(-max(DFA_CHUNK_FLOOR, int(dfa_chunk_bytes))
                                              // 64) * 64
