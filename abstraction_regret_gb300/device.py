@@ -178,21 +178,23 @@ SYMBOL_STATES = 1 << 15
 SYMBOL_PAIR_MEAN = 32.0
 
 
-def _closures(nfa) -> dict[int, np.ndarray]:
-    """The epsilon closure of every state that has epsilon edges."""
-    erp = np.asarray(nfa.eps_row_ptr, dtype=np.int64)
-    etg = np.asarray(nfa.eps_targets, dtype=np.int64)
-    out = {}
-    for s in np.flatnonzero(erp[1:] > erp[:-1]).tolist():
-        seen, todo = {s}, [s]
-        while todo:
-            u = todo.pop()
-            for t in etg[erp[u]:erp[u + 1]].tolist():
-                if t not in seen:
-                    seen.add(t)
-                    todo.append(t)
-        out[s] = np.fromiter(sorted(seen), dtype=np.int64, count=len(seen))
-    return out
+def _closures(nfa, weight: np.ndarray, limit: int):
+    """``(row int64[n + 1], states int32[])``: the epsilon closures of the start state and of
+    the states of positive ``weight`` that have epsilon edges; None when the sum of weight x
+    closure size passes ``limit``."""
+    n = int(nfa.num_states)
+    erp, etg = (np.ascontiguousarray(x, dtype=np.int32) for x in (nfa.eps_row_ptr,
+                                                                  nfa.eps_targets))
+    weight = np.ascontiguousarray(weight, dtype=np.int64)
+    row = np.zeros(n + 1, dtype=np.int64)
+    states = np.empty(limit + n, dtype=np.int32)
+    st = native.lib().gbfsm_eps_closures(
+        n, erp.ctypes.data, etg.ctypes.data if etg.size else None, weight.ctypes.data,
+        int(nfa.start_state), limit, row.ctypes.data, states.ctypes.data)
+    if st == native.UNSUPPORTED:
+        return None
+    native.check(st, "gbfsm_eps_closures")
+    return row, states
 
 
 def symbol_lists(nfa, limit: int = SYMBOL_LIST_LIMIT):
@@ -207,28 +209,34 @@ def symbol_lists(nfa, limit: int = SYMBOL_LIST_LIMIT):
     to = np.asarray(nfa.sym_targets, dtype=np.int64)
     src = np.repeat(np.arange(n, dtype=np.int64), np.diff(srp))
     wild = sym == ANY_SYMBOL
-    if int((~wild).sum()) + 256 * int(wild.sum()) > limit:
+    # pairs that a state's closure is multiplied by: one for an edge to it, 256 for a wildcard
+    weight = np.bincount(to, np.where(wild, 256, 1), n).astype(np.int64)
+    if int(weight.sum()) > limit:
         return None
-    closure = _closures(nfa)
-    if closure:  # edges to a state with epsilon edges lead to its closure
-        size = np.ones(n, dtype=np.int64)
-        for s, c in closure.items():
-            size[s] = c.size
-        count = size[to]
-        if int(count[~wild].sum()) + 256 * int(count[wild].sum()) > limit:
+    start = int(nfa.start_state)
+    first = np.array([start], dtype=np.int64)
+    if int(nfa.eps_row_ptr[-1]):  # edges to a state with epsilon edges lead to its closure
+        has_eps = np.diff(np.asarray(nfa.eps_row_ptr, dtype=np.int64)) > 0
+        found = _closures(nfa, weight, limit - int(weight[~has_eps].sum()))
+        if found is None:
             return None
-        more = np.flatnonzero(count > 1)
+        row, states = found
+        size = np.diff(row)
+        if size[start]:
+            first = states[row[start]:row[start + 1]].astype(np.int64)
+        more = np.flatnonzero(has_eps[to])
         if more.size:  # (these edges alone: an automaton has few of them)
-            one = count == 1
-            src = np.concatenate([src[one], np.repeat(src[more], count[more])])
-            sym = np.concatenate([sym[one], np.repeat(sym[more], count[more])])
-            to = np.concatenate([to[one]] + [closure[t] for t in to[more].tolist()])
+            one = ~has_eps[to]
+            count = size[to[more]]
+            at = np.repeat(row[to[more]] - np.cumsum(count) + count, count) + \
+                np.arange(int(count.sum()))
+            src = np.concatenate([src[one], np.repeat(src[more], count)])
+            sym = np.concatenate([sym[one], np.repeat(sym[more], count)])
+            to = np.concatenate([to[one], states[at].astype(np.int64)])
             wild = sym == ANY_SYMBOL
     c = np.concatenate([sym[~wild], np.repeat(np.arange(256), int(wild.sum()))])
     src = np.concatenate([src[~wild], np.tile(src[wild], 256)])
     to = np.concatenate([to[~wild], np.tile(to[wild], 256)])
-    start = int(nfa.start_state)
-    first = closure.get(start, np.array([start], dtype=np.int64))
     key = np.unique(np.concatenate([(c << 30) | (src << 15) | to, (256 << 30) | first]))
     row = np.searchsorted(key, np.arange(258, dtype=np.int64) << 30)
     acc = np.asarray(nfa.accept, dtype=bool)

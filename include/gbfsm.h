@@ -441,6 +441,15 @@ int32_t gbfsm_slots_build(int32_t num_states, const int32_t *sym_row_ptr,
                           int64_t cap_pairs, uint32_t *pairs, int64_t cap_codes,
                           uint32_t *codes, int64_t *info);
 
+/* The epsilon closures (host only, HOST arrays; csrc/closures.cu) of every state s that has
+ * epsilon edges and weight[s] > 0, and of `start`: states[row[s] .. row[s + 1]), s first, not
+ * sorted; empty for the others. row: [num_states + 1]; states: [limit + num_states].
+ * GBFSM_UNSUPPORTED as soon as the sum of weight[s] x closure size passes `limit`, or the
+ * epsilon edges followed pass a bound of about 64 x limit. No counterpart in the reference. */
+int32_t gbfsm_eps_closures(int32_t num_states, const int32_t *eps_row_ptr,
+                           const int32_t *eps_targets, const int64_t *weight, int32_t start,
+                           int64_t limit, int64_t *row, int32_t *states);
+
 /* Follow the set of all states of a DFA (HOST int32 [n * 256]) over `text` until it has at
  * most `want` members (host only; csrc/dfa_trial.cu). out[0] receives the bytes that took,
  * -1 when the text ended first or `schedules` times the lookups of a random DFA of as many
