@@ -176,6 +176,13 @@ SYMBOL_LIST_LIMIT = 256 * 1024  # pairs; 1024 to a byte on average
 SYMBOL_STATES = 1 << 15
 # automata that lanes run (two-byte supersets this small, engine.LANE_PAIR_MEAN) need none
 SYMBOL_PAIR_MEAN = 32.0
+# A step by the lists costs their length, one member by member the active states' edges. Up to
+# about SYMBOL_SHORT pairs a byte the lists are never slower; above, an edge to step over is
+# worth SYMBOL_EDGE pairs. Chunks of 64 inputs of 16 KiB, lists / member by member: 20000
+# states, 312 pairs a byte, one active state of 4 edges 0.89 / 0.88 ms; 328 pairs, 20 edges
+# 0.94 / 1.1; 875 pairs, 7 edges 2.9 / 1.1; 940 pairs, 30 edges 3.0 / 1.8; 60 edges 3.0 / 3.0.
+SYMBOL_SHORT = 300
+SYMBOL_EDGE = 14
 
 
 def _closures(nfa, weight: np.ndarray, limit: int):
@@ -243,6 +250,28 @@ def symbol_lists(nfa, limit: int = SYMBOL_LIST_LIMIT):
     src, to = (key >> 15) & 0x7FFF, key & 0x7FFF
     pairs = src | (to << 15) | (acc[to].astype(np.int64) << 30)
     return row.astype(np.uint32), pairs.astype(np.uint32)
+
+
+def symbol_lists_pay(nfa, row: np.ndarray, pairs: np.ndarray) -> bool:
+    """Whether warps should step by the symbol lists: short lists, or sets whose members have
+    many edges on trial texts (from all targets of a byte, as a chunk starts)."""
+    if int(row[256]) <= 256 * SYMBOL_SHORT:
+        return True
+    degree = np.diff(np.asarray(nfa.sym_row_ptr, dtype=np.int64))
+    enough = (int(row[256]) / 256 - SYMBOL_SHORT) / SYMBOL_EDGE + 12
+    src, to = pairs & 0x7FFF, (pairs >> 15) & 0x7FFF
+    start, steps = 8, 32  # bytes that a chunk's superset is given to shrink; bytes counted
+    for name in ("bytes", "lines"):
+        total, active = 0, None
+        for i, c in enumerate(_trial_texts()[name][: start + steps].tolist()):
+            a, b = int(row[c]), int(row[c + 1])
+            hit = to[a:b] if active is None else to[a:b][active[src[a:b]]]
+            active = np.zeros(degree.size, dtype=bool)
+            active[hit] = True
+            total += int(degree[active].sum()) if i >= start else 0
+        if total > enough * steps:
+            return True
+    return False
 
 
 def slot_table(nfa):
@@ -380,6 +409,8 @@ class DeviceNFA:
                     self._upload_lane_records(d, lane, precs[:, 0], ssy, nfa, dev)
             d.pair_row = self.pair_row.data_ptr()
         lists = symbol_lists(nfa) if self.pair_mean > SYMBOL_PAIR_MEAN else None
+        if lists is not None and not symbol_lists_pay(nfa, *lists):
+            lists = None
         self.sym_pairs = 0 if lists is None else int(lists[1].size)
         if lists is not None:
             with torch.cuda.device(dev):
