@@ -143,7 +143,7 @@ struct SlotRun {
 enum SlotEvent { kSlotAlive = 0, kSlotDead = 1, kSlotAccept = 2, kSlotFull = 3 };
 
 // One byte from any set: {one, m, event} of the next (kSlotFull: more members than a lane
-// holds). Out of line: a few bytes per chunk come here, and the loops that inline the
+// holds; set[0 .. m) is then still the set before the byte when it was that). Out of line: a few bytes per chunk come here, and the loops that inline the
 // common case stay small.
 template <typename Table>
 __device__ __noinline__ int3 slot_step_any(Table T, SlotCodes K, uint32_t one, int m,
@@ -160,8 +160,9 @@ __device__ __noinline__ int3 slot_step_any(Table T, SlotCodes K, uint32_t one, i
         int n = 0;
         for (int q = 0; q < m; ++q)
             if (T.look(set[q], c, next)) slot_add_code(T, K, out, n, next);
-        for (int q = 0; q < n && q < kSlotMembers; ++q) set[q] = out[q];
         m = n;
+        if (n <= kSlotMembers)
+            for (int q = 0; q < n; ++q) set[q] = out[q];
     }
     if (m == 0) return make_int3((int)K.multi_begin, 0, kSlotDead);
     if (m > kSlotMembers) return make_int3((int)K.multi_begin, 0, kSlotFull);
@@ -420,13 +421,14 @@ __device__ __forceinline__ bool slot_chunk(const gbfsm_nfa_dev &A, const Table &
 }
 
 // One lane: a whole input from the start state. False (no verdict) when a set outgrows the
-// lane.
+// lane: `at` is then the position before the byte that it does so on, and set[0 .. m) the set
+// there (m <= kSlotMembers codes of states).
 template <typename Table>
 __device__ __forceinline__ bool slot_whole(const gbfsm_nfa_dev &A, const Table &T,
-                                           const uint8_t *in, int64_t len, Verdict &v) {
+                                           const uint8_t *in, int64_t len, Verdict &v,
+                                           int64_t &at, uint32_t *set, int &m) {
     const SlotCodes K{A.set_code, A.accept_code, A.multi_code,
                       reinterpret_cast<const uint4 *>(A.code_recs)};
-    uint32_t set[kSlotMembers];
     SlotRun run{A.start_code, 1, set};
     v = Verdict{0, 0, len};
     if (A.start_code >= K.accept_begin) {
@@ -440,11 +442,20 @@ __device__ __forceinline__ bool slot_whole(const gbfsm_nfa_dev &A, const Table &
         uint32_t w = words.next_word();
         if (len - pos >= 4 && slot_word(T, K, run, w)) continue;
         for (int t = 0; t < 4 && pos + t < len; ++t, w >>= 8) {
+            const uint32_t one = run.one;
+            m = run.m;
             const int ev = slot_step(T, K, run, w & 0xffu);
             if (ev == kSlotAlive) continue;
-            if (ev == kSlotFull) return false;
-            const int64_t at = pos + t + 1;
-            v = ev == kSlotAccept ? Verdict{1, (int32_t)at, at} : Verdict{0, 0, at};
+            if (ev == kSlotFull) {
+                at = pos + t;
+                if (one != K.multi_begin) {
+                    m = 0;
+                    slot_add_code(T, K, set, m, one);
+                }
+                return false;
+            }
+            const int64_t end = pos + t + 1;
+            v = ev == kSlotAccept ? Verdict{1, (int32_t)end, end} : Verdict{0, 0, end};
             return true;
         }
     }

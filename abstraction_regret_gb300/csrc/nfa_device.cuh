@@ -552,6 +552,13 @@ struct WarpNfa {
         m = count;
     }
 
+    // The same, lane q < count holding the q-th record.
+    __device__ __forceinline__ void init_lane(const uint4 &rec, int count) {
+        mine = ((int)lane_id() < count) ? rec : make_uint4(0, 0, 0, 0);
+        mode = kReg;
+        m = count;
+    }
+
     // Write the current members' records to out[0 .. m) if there are at most `cap` of
     // them and they are listed (REG or LIST); returns m, or -1 if not written.
     __device__ int export_recs(uint4 *out, int cap) const {
@@ -602,25 +609,18 @@ struct BytesAhead {
     }
 };
 
-// Simulate one input with a whole warp, by stepper w (WarpNfa, or SymNfa of
-// sym_device.cuh). All lanes call it with identical arguments and all receive the verdict.
+// The rest of one input by a whole warp, from the set that stepper w (WarpNfa, or SymNfa of
+// sym_device.cuh) holds at position `pos`. All lanes call it with identical arguments and all
+// receive the verdict.
 template <typename Stepper>
-__device__ Verdict simulate_with(Stepper &w, const uint8_t *in, int64_t len) {
-    Verdict v{0, 0, 0};
-    int ev = w.init_start();
-    if (ev == kAccept) {
-        v.flag = 1;
-        w.cleanup();
-        return v;
-    }
+__device__ Verdict simulate_from(Stepper &w, const uint8_t *in, int64_t pos, int64_t len) {
+    Verdict v{0, 0, len};
     BytesAhead bytes;
-    bytes.init(in, len);
-    int64_t pos = 0;
-    v.examined = len;
+    bytes.init(in + pos, len - pos);
     while (pos < len) {
         ++pos;
         const uint32_t sym = bytes.advance();
-        ev = w.step(sym, bytes.next, bytes.next2);
+        const int ev = w.step(sym, bytes.next, bytes.next2);
         if (ev == kDead) {
             v.examined = pos;
             break;
@@ -634,6 +634,16 @@ __device__ Verdict simulate_with(Stepper &w, const uint8_t *in, int64_t len) {
     }
     w.cleanup();
     return v;
+}
+
+// Simulate one input with a whole warp, by stepper w.
+template <typename Stepper>
+__device__ Verdict simulate_with(Stepper &w, const uint8_t *in, int64_t len) {
+    if (w.init_start() == kAccept) {
+        w.cleanup();
+        return Verdict{1, 0, 0};
+    }
+    return simulate_from(w, in, 0, len);
 }
 
 // The same with the member-by-member stepper. `R` may point at shared-memory copies of the

@@ -43,6 +43,12 @@ __device__ __forceinline__ Rows global_rows(const gbfsm_nfa_dev &a) {
     return r;
 }
 
+// slot_whole() from global memory, out of line: the warp's steps after it need the registers.
+__device__ __noinline__ bool lane_whole(const gbfsm_nfa_dev &a, const uint8_t *in, int64_t len,
+                                        Verdict &v, int64_t &at, uint32_t *set, int &m) {
+    return slot_whole(a, GlobalSlots{a.slots, a.slot_pairs}, in, len, v, at, set, m);
+}
+
 template <bool kStaged>
 __global__ void __launch_bounds__(kMaxBlockThreads) nfa_warp_kernel(gbfsm_nfa_dev a, WarpPlan wp,
                                                         const uint8_t *__restrict__ data,
@@ -55,15 +61,22 @@ __global__ void __launch_bounds__(kMaxBlockThreads) nfa_warp_kernel(gbfsm_nfa_de
     const int input = (int)blockIdx.x * wp.warps_per_cta + warp;
     // A slot table: one lane walks the input with a lookup a byte (256 bytes on 1024 states:
     // 35 us against 120 us for the warp's steps, whose 8 lanes per member find one edge);
-    // the warp steps only inputs whose sets outgrow a lane, and nothing is staged when the
-    // CTA has none.
+    // the warp steps only inputs whose sets outgrow a lane, from the byte on which they do,
+    // and nothing is staged when the CTA has none.
     bool walked = input >= n_inputs;
+    int64_t from = 0;  // where the lane gave up, and the record of its set's lane-th member
+    int members = 0;
+    uint4 member = make_uint4(0, 0, 0, 0);
     if (a.slots != nullptr && wp.C > 0) {
+        uint32_t set[kSlotMembers];
         if (!walked && lane_id() == 0) {
             const int64_t b = offsets[input];
             Verdict v;
-            walked = slot_whole(a, GlobalSlots{a.slots, a.slot_pairs}, data + b,
-                                offsets[input + 1] - b, v);
+            int64_t at = 0;
+            int m = 0;
+            walked = lane_whole(a, data + b, offsets[input + 1] - b, v, at, set, m);
+            from = at;
+            members = m;
             if (walked) {
                 flags[input] = v.flag;
                 lens[input] = v.len;
@@ -71,7 +84,18 @@ __global__ void __launch_bounds__(kMaxBlockThreads) nfa_warp_kernel(gbfsm_nfa_de
             }
         }
         walked = __shfl_sync(GBFSM_FULL_MASK, walked ? 1 : 0, 0) != 0;
-        if (__syncthreads_and(walked)) return;
+        if (!walked) {
+            from = __shfl_sync(GBFSM_FULL_MASK, from, 0);
+            members = __shfl_sync(GBFSM_FULL_MASK, members, 0);
+            uint32_t code = 0;
+            for (int q = 0; q < members; ++q) {
+                const uint32_t c = __shfl_sync(GBFSM_FULL_MASK, lane_id() == 0 ? set[q] : 0u, 0);
+                if ((int)lane_id() == q) code = c;
+            }
+            if ((int)lane_id() < members)
+                member = __ldg(reinterpret_cast<const uint4 *>(a.code_recs) + code);
+        }
+        if (kStaged ? __syncthreads_and(walked) != 0 : walked) return;
     }
     Rows R;
     bool ok = true;
@@ -116,7 +140,15 @@ __global__ void __launch_bounds__(kMaxBlockThreads) nfa_warp_kernel(gbfsm_nfa_de
     zero_words(S.FB, W);
     __syncwarp();
     const int64_t b = offsets[input];
-    const Verdict v = simulate_warp<kStaged>(a, R, data + b, offsets[input + 1] - b, S);
+    const int64_t len = offsets[input + 1] - b;
+    Verdict v{1, 0, 0};
+    WarpNfa<kStaged> w(a, R, S);
+    bool alive = true;
+    if (members > 0)
+        w.init_lane(member, members);
+    else
+        alive = w.init_start() != kAccept;
+    if (alive) v = simulate_from(w, data + b, from, len);
     if (lane_id() == 0) {
         flags[input] = v.flag;
         lens[input] = v.len;
