@@ -202,13 +202,12 @@ __device__ inline void run_chunk(const gbfsm_nfa_dev &nfa, const Rows &R, WarpSc
         }
     }
     const int64_t len = e - b;
-    BytesAhead bytes;
+    typename Stepper::Bytes bytes;
     bytes.init(base + b, stopped ? 0 : len);
     int64_t j = 0;
     while (!stopped && j < len) {
         ++j;
-        const uint32_t sym = bytes.advance();
-        ev = w.step(sym, bytes.next, bytes.next2);
+        ev = w.next_step(bytes);
         const int32_t pos = (int32_t)(b + j);
         if (ev == kDead) {
             dead_at = pos;

@@ -494,10 +494,11 @@ struct WarpNfa {
         return (info & GBFSM_EDGE_ACCEPT) ? kAccept : kAlive;
     }
 
-    // (the bytes after, `next` and `next2`, are for steppers that load ahead)
-    __device__ __forceinline__ int step(uint32_t sym, int next = -1, int next2 = -1) {
-        (void)next;
-        (void)next2;
+    using Bytes = ByteStream;  // what next_step() reads
+
+    __device__ __forceinline__ int next_step(Bytes &bytes) { return step(bytes.next()); }
+
+    __device__ __forceinline__ int step(uint32_t sym) {
         return mode == kReg ? step_reg(sym) : step_general(sym);
     }
 
@@ -585,42 +586,17 @@ struct WarpNfa {
     }
 };
 
-// A byte stream with the two bytes after the current one (-1 past the end).
-struct BytesAhead {
-    ByteStream bytes;
-    int64_t left;  // bytes not yet taken from the stream
-    int now, next, next2;
-
-    __device__ __forceinline__ int take() { return left > 0 ? (--left, (int)bytes.next()) : -1; }
-
-    __device__ __forceinline__ void init(const uint8_t *in, int64_t len) {
-        bytes.init(in, len);
-        left = len;
-        now = -1;
-        next = take();
-        next2 = take();
-    }
-
-    __device__ __forceinline__ uint32_t advance() {
-        now = next;
-        next = next2;
-        next2 = take();
-        return (uint32_t)now;
-    }
-};
-
 // The rest of one input by a whole warp, from the set that stepper w (WarpNfa, or SymNfa of
 // sym_device.cuh) holds at position `pos`. All lanes call it with identical arguments and all
 // receive the verdict.
 template <typename Stepper>
 __device__ Verdict simulate_from(Stepper &w, const uint8_t *in, int64_t pos, int64_t len) {
     Verdict v{0, 0, len};
-    BytesAhead bytes;
+    typename Stepper::Bytes bytes;
     bytes.init(in + pos, len - pos);
     while (pos < len) {
         ++pos;
-        const uint32_t sym = bytes.advance();
-        const int ev = w.step(sym, bytes.next, bytes.next2);
+        const int ev = w.next_step(bytes);
         if (ev == kDead) {
             v.examined = pos;
             break;

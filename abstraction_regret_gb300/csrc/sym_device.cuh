@@ -32,6 +32,29 @@ __device__ __forceinline__ bool sym_usable(const gbfsm_nfa_dev &A, int list_capa
            A.num_words * 8 <= 32 * max(list_capacity, 32);
 }
 
+// A byte stream with the two bytes after the current one (-1 past the end).
+struct BytesAhead {
+    ByteStream bytes;
+    int64_t left;  // bytes not yet taken from the stream
+    int next, next2;
+
+    __device__ __forceinline__ int take() { return left > 0 ? (--left, (int)bytes.next()) : -1; }
+
+    __device__ __forceinline__ void init(const uint8_t *in, int64_t len) {
+        bytes.init(in, len);
+        left = len;
+        next = take();
+        next2 = take();
+    }
+
+    __device__ __forceinline__ int advance() {
+        const int now = next;
+        next = next2;
+        next2 = take();
+        return now;
+    }
+};
+
 struct SymNfa {
     const gbfsm_nfa_dev &A;
     uint32_t *cur;  // the set; the other bitmap is all zero between steps
@@ -116,8 +139,13 @@ struct SymNfa {
     // The superset of a chunk start: whatever the set was before byte c.
     __device__ __forceinline__ int init_after(uint32_t c) { return advance((int)c, true, -1, -1); }
 
-    __device__ __forceinline__ int step(uint32_t sym, int next = -1, int next2 = -1) {
-        return advance((int)sym, false, next, next2);
+    __device__ __forceinline__ int step(uint32_t sym) { return advance((int)sym, false, -1, -1); }
+
+    using Bytes = BytesAhead;  // what next_step() reads
+
+    __device__ __forceinline__ int next_step(Bytes &bytes) {
+        const int sym = bytes.advance();
+        return advance(sym, false, bytes.next, bytes.next2);
     }
 
     __device__ __forceinline__ int count() const {
