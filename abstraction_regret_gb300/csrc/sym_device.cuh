@@ -156,15 +156,6 @@ struct SymNfa {
         return c;
     }
 
-    // Start from state records (distinct states, closed under epsilon, count <= 32).
-    __device__ __forceinline__ void init_recs(const uint4 *recs, int count) {
-        if ((int)lane_id() < count) {
-            const uint32_t s = recs[lane_id()].x;
-            atomicOr(cur + (s >> 5), 1u << (s & 31u));
-        }
-        __syncwarp();
-    }
-
     // The members' records to out[0 .. m) when there are at most `cap`; m, or -1.
     __device__ __forceinline__ int export_recs(uint4 *out, int cap) const {
         const int m = count();
