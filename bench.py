@@ -10,7 +10,8 @@ that keep the active set alive and no accepting state, so every offered byte is
 examined (the literal configuration's uniform bytes kill the active set after about one
 byte). Inputs are larger than L2 (261 MB > 129 MB).
 
-Printed (rank 0, one JSON line):
+Printed (rank 0): one JSON line with the headline, its roofline and baseline and the serving
+percentiles on standard output; the same with every section in full on standard error:
   value       GB/s of input through the engine's launches (lane launch, persistent
               launch, overflow pass, fix-up), inputs resident in HBM (CUDA events
               around K steps on the launching stream);
@@ -313,6 +314,38 @@ def attach_rooflines(extras: dict, onchip: dict | None, hbm: float) -> None:
             v["roofline"].update(dfa_roofline(c["examined"], c["chains"], v["ms"], onchip, hbm))
 
 
+# what the printed line holds of a section (None: all of it)
+HEADLINE = {
+    "metric": None, "value": None, "unit": None, "n_gpus": None, "steps": None, "warmup": None,
+    "ms_per_step": None, "higher_is_better": None, "scaling": None, "vs_baseline": None,
+    "dtype": None, "data": None, "config": None, "gpu_launches": None, "clocks": None,
+    "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "ms_per_step"),
+    "oracle_gate": ("checked", "accepted"),
+    "roofline": ("bound", "achieved", "peak", "unit", "frac", "traffic", "peak_source", "kernel",
+                 "kernel_ms"),
+    "cpu_baseline": None,
+    "speedup_vs_plain_per_input": None, "speedup_vs_plain_single_launch": None,
+}
+
+
+def headline(line: dict) -> dict:
+    """The short form of the result, which is printed: every contracted key, and the serving
+    percentiles. With all sections in it the line grew to more than its readers take."""
+    out = {}
+    for key, parts in HEADLINE.items():
+        if key in line:
+            v = line[key]
+            out[key] = {k: v[k] for k in parts if k in v} if parts and isinstance(v, dict) else v
+    traces = {"literal": line.get("serving", {}).get("rates", [])}
+    for name, t in line.get("serving", {}).get("examined_traces", {}).items():
+        traces[name] = t.get("rates", [])
+    if any(traces.values()):
+        out["serving"] = {name: [{"rate_per_s": r["rate_per_s"], "p50_ms": round(r["p50_ms"], 3),
+                                  "p99_ms": round(r["p99_ms"], 3)} for r in rates]
+                          for name, rates in traces.items()}
+    return out
+
+
 def cpu_reference(batch, budget_s: float = 15.0, threads: int | None = None):
     """The oracle port on this host's cores: whole passes over the batch (inputs spread
     over all threads) until ``budget_s`` of wall time has gone; at least one pass."""
@@ -536,7 +569,8 @@ def main(argv=None) -> int:
             # per examined symbol: 1 input byte (HBM stream) + one 2-byte table entry read
             # from on-chip memory; an input is one chain of dependent lookups, or two where
             # the launch cuts it (a DFA that rarely accepts)
-            chains2 = int(b2.n_inputs) * (2 if ex2.dev.desc.flags else 1)
+            cut = native.DFA_RARE_ACCEPT | native.DFA_COLLAPSES
+            chains2 = int(b2.n_inputs) * (2 if ex2.dev.desc.flags & cut == cut else 1)
             longest = int(np.diff(b2.offsets).max())
             extras[f"dfa_c2_{variant}"] = {
                 "offered_GBps": b2.total_bytes / (d_ms * 1e-3) / 1e9,
@@ -681,7 +715,8 @@ def main(argv=None) -> int:
                 "oracle_gate": gate,
                 "roofline": roofline, "cpu_baseline": cpu, "clocks": clk.summary()}
         line.update(extras)
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(headline(line)), flush=True)
     if world > 1:
         dist.destroy_process_group()
     return 0
