@@ -247,3 +247,34 @@ def test_slow_collapses_end_in_their_chunks(states, share):
     p = eng._dplan.records[: n * native.CHUNK_RECORD_BYTES].cpu().numpy().view(np.int32) \
         .reshape(n, -1)[:, 0]
     assert n >= 8 and (p >= 0).mean() > 0.95
+
+
+def test_texts_that_the_trial_did_not_foresee():
+    """Bytes 0 and 1 permute the states and every other byte leads to state 0, so the set falls
+    together on every trial text but never on these inputs: collapses run out of budget, the
+    plain launch's (which cuts the inputs) and the engine's."""
+    import torch
+
+    from abstraction_regret_gb300 import native
+    from abstraction_regret_gb300.engine import GraphRunner
+    from abstraction_regret_gb300.executors import CudaDFAExecutor
+
+    dfa = _permuting(4096, 13, (0, 1))
+    rng = np.random.default_rng(14)
+    inputs = []
+    for k in range(64):
+        x = rng.integers(0, 2, (16384, 16384, 16383, 9000)[k % 4], dtype=np.uint8)
+        if k % 3 == 0:
+            x[int(rng.integers(0, x.size))] = 48
+        inputs.append(x.tobytes())
+    _plain(dfa, inputs)
+    _check(dfa, inputs)
+    ex = CudaDFAExecutor(dfa)
+    assert ex.dev.desc.flags == native.DFA_RARE_ACCEPT | native.DFA_COLLAPSES
+    data, off = O.flatten(inputs)
+    d = torch.from_numpy(np.concatenate([data, np.zeros(16, np.uint8)])).cuda()
+    o = torch.from_numpy(off).cuda()
+    out = torch.zeros((3, len(inputs)), dtype=torch.int32, device="cuda")
+    assert _ms(lambda: ex.launch(d, o, len(inputs), out[0], out[1], out[2])) < 16384 * 0.3e-3 * 2
+    runner = GraphRunner(PersistentEngine([dfa]), [0] * len(inputs), data, off)
+    assert _ms(runner.kernel_only) < 16384 * 0.3e-3 * 2
