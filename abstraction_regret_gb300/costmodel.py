@@ -109,9 +109,11 @@ def traffic_per_symbol(f, technique: str, threads: int = 128, staged: bool = Fal
 class CostModel:
     """The effective bandwidth of modelled traffic and the time of one dependent step of
     a chain (one symbol of one input) -- the two constants ``fit`` estimates -- plus the
-    engine's per-lane step times, launch overhead and lane count (measured on GB300:
-    the c3 lane launch, 1728-byte chunks in 1.83 ms; one warp per input, 575 ms for a
-    1 MiB input)."""
+    engine's per-lane step times, launch overhead and lane count. The step times are those of
+    sets stepped member by member (measured on GB300: 16384 states, 1728-byte lane chunks in
+    1.83 ms; one warp per input, 575 ms for a 1 MiB input). Automata with a slot table take
+    0.05-0.17 us a plain step and 0.22 us a lane step; held against each other the two
+    predictions then turn to the engine somewhat early, from a few hundred bytes an input."""
 
     eff_bandwidth_bytes_per_s: float = 4.0e12
     step_s: float = 5.5e-7            # plain launch: one warp's step on one input

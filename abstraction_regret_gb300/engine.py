@@ -69,7 +69,7 @@ LANE_WARPS_PER_SM = 32
 # so the shortest one is half as long again. A DFA whose set did not shrink on trial is cut
 # into chunks of at least DFA_CHUNK_LONG bytes and DFA_CHUNK_LONG_STATES bytes a state, and
 # its shorter inputs run whole: 64 inputs of 16 KiB on 4096 permuted states took 34.8 ms in
-# chunks of 1344 bytes and take 3.5 whole. So is a DFA that accepts every
+# chunks of 1344 bytes and take 2.8 whole. So is a DFA that accepts every
 # DFA_OFTEN_BYTES bytes on average, whose inputs all but end within the 4096 bytes that their
 # first chunk walks before anything else: the other chunks' collapses are for nothing (0.5% of
 # the entries accepting, 300 inputs of up to 4 MiB 1.13 ms in short chunks, 0.75 in long ones;

@@ -515,7 +515,7 @@ gbfsm_status gbfsm_lanes_run_range(const gbfsm_automaton *table, int32_t n_autom
                                   (the automaton needs first_row / first_edges) */
 #define GBFSM_PLAN_NFA_LANES 2 /* NFA: every input cut into lane chunks (the automaton
                                   needs the lane tables) */
-#define GBFSM_PLAN_DFA 3       /* DFA inputs, 32 per task, one walk per lane; inputs of at
+#define GBFSM_PLAN_DFA 3       /* DFA inputs, up to 32 per task, one walk per lane; inputs of at
                                   least two DFA chunks (gbfsm_batch_plan_args.aut_dfa_chunk,
                                   dfa_warps) are cut into DFA chunks instead */
 
