@@ -501,15 +501,23 @@ COLLAPSE_SCHEDULES = 32
 SPLIT_SCHEDULES = 2
 
 
+TRIAL_TEXTS = ("bytes", "lines", "digits")
+
+
 @lru_cache(maxsize=1)
 def _trial_texts() -> dict[str, np.ndarray]:
     """Texts on which a DFA's set of all states is tried: any bytes, lines of printable
     ones, and digits (a counter over digits leaves every other byte to a sink, so that on
-    any other text its states fall together at once)."""
-    any_byte, a, b = np.frombuffer(np.random.default_rng(20).bytes(3 << 15),
-                                   dtype=np.uint8).reshape(3, -1)
+    any other text its states fall together at once). Rows of one array."""
+    # (SplitMix64 counters; numpy's own generator takes 8 ms to come up)
+    z = np.arange(1, (3 << 15) // 8 + 1, dtype=np.uint64) * np.uint64(0x9E3779B97F4A7C15)
+    z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+    z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+    out = (z ^ (z >> np.uint64(31))).view(np.uint8).reshape(3, -1).copy()
     line = np.concatenate([32 + np.arange(252) % 95, [10] * 4]).astype(np.uint8)
-    return {"bytes": any_byte, "lines": line[a], "digits": (48 + b % 10).astype(np.uint8)}
+    out[1] = line[out[1]]
+    out[2] = 48 + out[2] % 10
+    return dict(zip(TRIAL_TEXTS, out))
 
 
 def collapse_trial(dfa) -> dict[str, tuple[int, float, int]]:
@@ -518,16 +526,18 @@ def collapse_trial(dfa) -> dict[str, tuple[int, float, int]]:
     that a random DFA's takes, SPLIT_SCHEDULES times for digits), the lookups as a multiple of
     a random DFA's, and the lookups. Up to the first text on which it has not."""
     trans = np.ascontiguousarray(dfa.trans, dtype=np.int32)
-    out = np.zeros(3, dtype=np.int64)
+    texts = _trial_texts()
+    schedules = np.array([SPLIT_SCHEDULES if name == "digits" else COLLAPSE_SCHEDULES
+                          for name in TRIAL_TEXTS], dtype=np.int32)
+    out = np.zeros((3, 3), dtype=np.int64)
+    st = native.lib().gbfsm_dfa_collapse_trial(
+        int(dfa.num_states), trans.ctypes.data, texts["bytes"].ctypes.data, len(TRIAL_TEXTS),
+        texts["bytes"].size, DFA_ENTRY_STATES, schedules.ctypes.data, out.ctypes.data)
+    native.check(st, "gbfsm_dfa_collapse_trial")
     found = {}
-    for name, text in _trial_texts().items():
-        st = native.lib().gbfsm_dfa_collapse_trial(
-            int(dfa.num_states), trans.ctypes.data, text.ctypes.data, text.size,
-            DFA_ENTRY_STATES, SPLIT_SCHEDULES if name == "digits" else COLLAPSE_SCHEDULES,
-            out.ctypes.data)
-        native.check(st, "gbfsm_dfa_collapse_trial")
-        found[name] = (int(out[0]), int(out[1]) / int(out[2]), int(out[1]))
-        if found[name][0] < 0:
+    for name, (end, lookups, random) in zip(TRIAL_TEXTS, out.tolist()):
+        found[name] = (end, lookups / random, lookups)
+        if end < 0:
             break
     return found
 

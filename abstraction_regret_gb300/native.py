@@ -238,7 +238,7 @@ SIGNATURES: dict[str, tuple] = {
     "gbfsm_slots_build": (_i32, [_i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _i64, _vp,
                                  _vp]),
     "gbfsm_eps_closures": (_i32, [_i32, _vp, _vp, _vp, _i32, _i64, _vp, _vp]),
-    "gbfsm_dfa_collapse_trial": (_i32, [_i32, _vp, _vp, _i64, _i32, _i32, _vp]),
+    "gbfsm_dfa_collapse_trial": (_i32, [_i32, _vp, _vp, _i32, _i64, _i32, _vp, _vp]),
     "gbfsm_lanes_stage_limit": (_i32, []),
     "gbfsm_sym_fixup_run": (ctypes.c_int, [_vp, _i32, _i32, _vp, _i32, _vp, _vp, _vp,
                                            _P(ChunkIO), _P(Plan), _vp, _vp, _vp, _vp]),

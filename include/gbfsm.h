@@ -450,13 +450,15 @@ int32_t gbfsm_eps_closures(int32_t num_states, const int32_t *eps_row_ptr,
                            const int32_t *eps_targets, const int64_t *weight, int32_t start,
                            int64_t limit, int64_t *row, int32_t *states);
 
-/* Follow the set of all states of a DFA (HOST int32 [n * 256]) over `text` until it has at
- * most `want` members (host only; csrc/dfa_trial.cu). out[0] receives the bytes that took,
- * -1 when the text ended first or `schedules` times the lookups of a random DFA of as many
- * states were not enough; out[1] the table lookups made, out[2] a random DFA's (want 16).
- * No counterpart in the reference. */
-int32_t gbfsm_dfa_collapse_trial(int32_t num_states, const int32_t *trans, const uint8_t *text,
-                                 int64_t len, int32_t want, int32_t schedules, int64_t *out);
+/* Follow the set of all states of a DFA (HOST int32 [n * 256]) over each of n_texts (1..8)
+ * texts of len bytes, one after the other in `texts`, until it has at most `want` members
+ * (host only, a thread per text for large DFAs; csrc/dfa_trial.cu). For text k out[3k]
+ * receives the bytes that took, -1 when the text ended first or schedules[k] times the
+ * lookups of a random DFA of as many states were not enough; out[3k + 1] the table lookups
+ * made, out[3k + 2] a random DFA's (want 16). No counterpart in the reference. */
+int32_t gbfsm_dfa_collapse_trial(int32_t num_states, const int32_t *trans, const uint8_t *texts,
+                                 int32_t n_texts, int64_t len, int32_t want,
+                                 const int32_t *schedules, int64_t *out);
 
 /* Largest gbfsm_chunk_io.lane_stage_bytes of the lane launch on the current device. */
 int32_t gbfsm_lanes_stage_limit(void);

@@ -72,9 +72,12 @@ def test_bad_tables_are_refused():
     dfa.trans[:] = 20
     with pytest.raises(ValueError):
         D.collapse_trial(dfa)
-    lib, out = native.lib(), np.zeros(3, np.int64)
-    assert lib.gbfsm_dfa_collapse_trial(0, None, None, 0, 16, 8, out.ctypes.data) == \
-        native.INVALID_ARG
+    lib, out, one = native.lib(), np.zeros(3, np.int64), np.ones(1, np.int32)
+    text = np.zeros(16, np.uint8)
+    for states, texts in ((0, 1), (20, 0), (20, 9)):
+        assert lib.gbfsm_dfa_collapse_trial(
+            states, dfa.trans.ctypes.data, text.ctypes.data, texts, 1, 16, one.ctypes.data,
+            out.ctypes.data) == native.INVALID_ARG
 
 
 def _lazy(n, share, seed=1):
