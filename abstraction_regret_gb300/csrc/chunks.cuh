@@ -836,11 +836,11 @@ __device__ inline Verdict serial_fixup(WarpNfa<false> &w, const uint8_t *base, i
 
 // One warp: the link scan over an input's chunk records, 128 chunks a round, four per lane,
 // whose records are loaded together (the scan waits for its loads: the fix-up of 24 inputs of
-// up to 1 MiB, 4096 chunks, takes 62 us, 107 at 32 chunks a round). True when it
+// up to 1 MiB, 4096 chunks, takes 58 us, 107 at 32 chunks a round). True when it
 // decides the input (v); else last_rec is the last chunk whose recorded end set is exact (-1:
-// not even the first's). Out of line: the views need the registers that the steppers around
-// it hold.
-static __device__ __noinline__ bool scan_links(const ChunkRecord *recs, int first, int count,
+// not even the first's). Inlined: as a call it cost the persistent kernel's steppers their
+// registers (92 bytes spilled, now none; chunks stepped member by member 1.00 ms, now 0.98).
+__device__ __forceinline__ bool scan_links(const ChunkRecord *recs, int first, int count,
                                                Verdict &v, int &last_rec) {
     constexpr int kRounds = 4;
     const uint32_t lane = lane_id();
